@@ -5,6 +5,7 @@ Every translation unit under csrc/ is compiled separately (in parallel) with
 shared object exposing the C ABI of include/boris_b200.h.
 """
 import os
+import re
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -33,13 +34,25 @@ def _compile(src, extra):
     return obj, r.stderr
 
 
-def _stale(src, hdr_mtime, force):
+def _includes(path, seen):
+    """The project headers a file includes, itself first, recursively."""
+    if path in seen or not os.path.exists(path):
+        return seen
+    seen.add(path)
+    with open(path) as f:
+        for name in re.findall(r'^\s*#include "([^"]+)"', f.read(), re.M):
+            for d in (CSRC, os.path.join(HERE, "..", "include")):
+                _includes(os.path.join(d, name), seen)
+    return seen
+
+
+def _stale(src, force):
     """A translation unit is recompiled when forced, when its object is missing, or when the object is
-    older than the source or than the newest shared header / build recipe."""
+    older than the source, a header it includes or the build recipe."""
     obj = os.path.join(OBJDIR, src + ".o")
     if force or not os.path.exists(obj):
         return True
-    return os.path.getmtime(obj) < max(os.path.getmtime(os.path.join(CSRC, src)), hdr_mtime)
+    return os.path.getmtime(obj) < max(os.path.getmtime(p) for p in _includes(os.path.join(CSRC, src), set()) | {__file__})
 
 
 def build(force=False, verbose=False, extra=None):
@@ -47,10 +60,7 @@ def build(force=False, verbose=False, extra=None):
     extra = list(extra or [])
     os.makedirs(LIBDIR, exist_ok=True)
     os.makedirs(OBJDIR, exist_ok=True)
-    hdr = os.path.join(HERE, "..", "include", "boris_b200.h")
-    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith((".cu", ".cpp"))]
-    hdr_mtime = max([os.path.getmtime(h) for h in headers] + [os.path.getmtime(hdr), os.path.getmtime(__file__)])
-    todo = [s for s in _sources() if extra or _stale(s, hdr_mtime, force)]
+    todo = [s for s in _sources() if extra or _stale(s, force)]
     objs = [os.path.join(OBJDIR, s + ".o") for s in _sources()]
     if not todo and os.path.exists(LIB) and os.path.getmtime(LIB) >= max(os.path.getmtime(o) for o in objs):
         return LIB

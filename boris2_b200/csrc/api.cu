@@ -1387,7 +1387,7 @@ int yz_multi(bm_ctx *c, int gate, int *count)
             if (ypass_has_reg(m.Ny)) {
                 while (W > 1 && (ymid2d_reg_threads(m.Ny, W) > 384 || ymid2d_smem<T>(m.Ny, W) > 100 * 1024 || W > m.LX)) W /= 2;
                 a.W = W;
-                g2[m.Ny].push_back(a);
+                g2[m.Ny % 3 ? m.Ny : 3].push_back(a);
             } else {
                 while (W > 1 && (W * m.py.tpl > lim || ymid2d_smem<T>(m.Ny, W) > 100 * 1024 || W > m.LX)) W /= 2;
                 a.W = W;
@@ -1397,7 +1397,7 @@ int yz_multi(bm_ctx *c, int gate, int *count)
         }
         int Wy, Wz;
         batch_tiles<T>(m, Wy, Wz);
-        if (ypass_has_reg(m.Ny)) {
+        if (ypass_has_reg(m.Ny) && !(m.Ny % 3 == 0 && ypass_has_st(m.Ny))) {
             int W = 16;
             while (W > 1 && (ypass_reg_threads(m.Ny, W) > std::min(lim, yreg_maxt<T>::v) || (size_t)m.Ny * W * sizeof(cpx<T>) > 64 * 1024 ||
                              W > m.LX)) W /= 2;

@@ -218,7 +218,7 @@ template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s);
 #define BM_BATCH_ZMID_REG 5   // key Nz
 #define BM_BATCH_YFWD_REG 6   // key Ny
 #define BM_BATCH_YINV_REG 7   // key Ny
-#define BM_BATCH_YMID2D_REG 8 // key Ny
+#define BM_BATCH_YMID2D_REG 8 // key Ny (powers of two), or 3: every 3 * 2^k length together
 #define BM_BATCH_YFWD_ST 9    // key Ny (Stockham y transform)
 #define BM_BATCH_YINV_ST 10   // key Ny
 template <typename T>
