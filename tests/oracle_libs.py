@@ -22,7 +22,13 @@ REF_SO = os.path.join(ORACLE_DIR, "_ref", "libborisref.so")
 
 def _reference_tree():
     """Root of the reference source tree: $BORIS2_REFERENCE, else the default of oracle/Makefile's
-    REF variable (the one recipe that names where the reference is mounted)."""
+    REF variable (the one recipe that names where the reference is mounted); "" when that root holds no
+    sources."""
+    root = _reference_root()
+    return root if os.path.isdir(os.path.join(root, "Boris")) else ""
+
+
+def _reference_root():
     env = os.environ.get("BORIS2_REFERENCE")
     if env:
         return env
