@@ -122,6 +122,7 @@ struct BatchRec {
     int key;              // register-kernel length of the launch (0: generic-length kernel)
     size_t args_off, work_off;
     int nwork, nt;
+    unsigned int total = 0;   // stage launches: work items of the set's launches together
     size_t smem;
     int plain = 0;        // stage launch: every argument block is a plain stage update (stage_plain)
 };
@@ -154,6 +155,8 @@ struct LaunchTimer {
 struct bm_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    std::vector<cudaStream_t> side;       // side streams of the batched step's independent launches (Branches)
+    std::vector<cudaEvent_t> side_ev;     // fork / join events of the capture in progress
     int precision = BM_MIXED;
     int eval = BM_RK4;
     double dt = 1e-13;
@@ -506,11 +509,28 @@ float time_launches(cudaStream_t s, F launch, int reps)
     cudaEventSynchronize(e1);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
+    ms /= reps;
+    if (ms < 0.05f) {
+        // launches of a few microseconds: a longer run, the better of the two (3 launches alone picked
+        // stage shapes twice as slow as the best on small films)
+        const int more = 4 * reps;
+        cudaEventRecord(e0, s);
+        for (int r = 0; r < more; r++) launch();
+        cudaEventRecord(e1, s);
+        cudaEventSynchronize(e1);
+        float m2 = 0.f;
+        cudaEventElapsedTime(&m2, e0, e1);
+        ms = std::min(ms, m2 / more);
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (cudaGetLastError() != cudaSuccess) return 1e30f;
-    return ms / reps;
+    return ms;
 }
+
+// Row counts per block the stage tuner tries: 1, and more while at least one block per SM remains (fewer
+// blocks only leave SMs idle: 7 blocks of 480 threads took 21 us where 64 blocks of one row took 10)
+bool tune_rows_ok(int rows, int rpb) { return rpb == 1 || (rows + rpb - 1) / rpb >= 148; }
 
 // 3D y passes of one grid: transform variant (two-level register / radix-16 Stockham) x column
 // tile width, timed as a forward + inverse pair on the grid's own spectra
@@ -580,7 +600,7 @@ int tune_grid_x(bm_ctx *c, Mesh &G)
     for (int xv = 0; xv <= (stage_reg_q(G.LX, 2) ? (sizeof(T) == 4 ? 3 : 2) : 1); xv++)
         for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
             const int tpl = stage_reg_q(G.LX, xv) ? stage_reg_q(G.LX, xv) : G.px.tpl;
-            if (((3 * rpb * tpl + 31) & ~31) > lim) break;
+            if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
             if ((size_t)3 * rpb * padded_len(G.LX) * cs > 200 * 1024) break;
             f.rpb = h.rpb = rpb;
             f.xv = h.xv = xv;
@@ -682,7 +702,7 @@ int autotune_mesh(bm_ctx *c, Mesh &m)
             for (int stg = 0; stg <= (reg ? 1 : 0); stg++)
                 for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
                     const int tpl = stage_reg_q(m.LX, xv) ? stage_reg_q(m.LX, xv) : m.px.tpl;
-                    if (((3 * rpb * tpl + 31) & ~31) > lim) break;
+                    if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
                     if ((size_t)3 * rpb * padded_len(m.LX) * cs > 200 * 1024) break;
                     a.rpb = rpb;
                     a.staged = stg;
@@ -1205,6 +1225,64 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
 template <typename T> T *B(Mesh &m, int i) { return (T *)m.buf[i]; }
 template <typename T> T *E(Mesh &m, int i) { return (T *)m.ev[i]; }
 
+// Independent launches of a captured batched step as parallel branches of its graph: next() moves the
+// context to another side stream that waits for the fork point, join() brings the work back to the main
+// stream. The launches of one pass of a batch (one per transform length) touch different meshes, and most
+// of them fill a fraction of the GPU (48 .. 180 blocks), so one after another they leave it idle: 24 uneven
+// films took 3.13 ms of summed kernel time per RK4 step.
+struct Branches {
+    bm_ctx *c;
+    cudaStream_t main;
+    cudaEvent_t fork = nullptr;
+    int used = 0, turn = 0;
+    explicit Branches(bm_ctx *ctx) : c(ctx), main(ctx->stream) {}
+    cudaEvent_t event()
+    {
+        cudaEvent_t e = nullptr;
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return nullptr;
+        c->side_ev.push_back(e);
+        return e;
+    }
+    // the stream of the next independent launch; the first one stays on the main stream
+    int next()
+    {
+        if (c->bp.collect) return 0;
+        if (!fork) {
+            if (!(fork = event())) return fail(BM_ECUDA, "branch event");
+            CK(cudaEventRecord(fork, main));
+            return 0;
+        }
+        const int k = turn++ % kSide;
+        while ((int)c->side.size() <= k) {
+            cudaStream_t s = nullptr;
+            CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+            c->side.push_back(s);
+        }
+        if (k >= used) {
+            CK(cudaStreamWaitEvent(c->side[k], fork, 0));
+            used = k + 1;
+        }
+        c->stream = c->side[k];
+        return 0;
+    }
+    int join()
+    {
+        c->stream = main;
+        for (int k = 0; k < used; k++) {
+            cudaEvent_t e = event();
+            if (!e) return fail(BM_ECUDA, "branch event");
+            CK(cudaEventRecord(e, c->side[k]));
+            CK(cudaStreamWaitEvent(main, e, 0));
+        }
+        used = turn = 0;
+        fork = nullptr;
+        return 0;
+    }
+    // an error path leaves the context on its own stream
+    ~Branches() { c->stream = main; }
+    static constexpr int kSide = 7;
+};
+
 // ------------------------------------------------------------------ many meshes per launch
 size_t bp_append(BatchPlan &bp, const void *p, size_t bytes)
 {
@@ -1217,8 +1295,8 @@ size_t bp_append(BatchPlan &bp, const void *p, size_t bytes)
 // stage kernels of several meshes: per-mesh launches, or one launch over (mesh, row block) items
 // with the generic-length kernel (rows per block chosen so every mesh fills ~256 threads)
 // stage kernels of every mesh: one launch per x length with a radix-8 register kernel, one for
-// the remaining lengths (generic kernel). Only the last launch finishes the step (error-norm
-// controller, time advance); the earlier ones only add to the error-norm maximum.
+// the remaining lengths (generic kernel), as parallel branches. The last work item of the set's launches
+// finishes the step (error-norm controller, time advance).
 template <typename T>
 int stage_batch_one(bm_ctx *c, int key, std::vector<StageArgs<T>> &v, int *count)
 {
@@ -1260,7 +1338,7 @@ int stage_batch_one(bm_ctx *c, int key, std::vector<StageArgs<T>> &v, int *count
     const BatchRec &r = bp.recs[bp.next++];
     const char *base = (const char *)bp.dbuf;
     CKL(launch_stage_batch<T>(r.key, (const StageArgs<T> *)(base + r.args_off), (const int2 *)(base + r.work_off), r.nwork,
-                              r.nt, r.smem, c->stream, r.plain), "stage batch");
+                              r.total, r.nt, r.smem, c->stream, r.plain), "stage batch");
     (*count)++;
     return 0;
 }
@@ -1282,16 +1360,24 @@ int stage_multi(bm_ctx *c, std::vector<StageArgs<T>> &v, int *count)
     int lk = BM_LAST_NONE, pub = 0;
     for (auto &a : v) if (a.last_kind != BM_LAST_NONE) lk = a.last_kind;
     for (auto &a : v) if (a.diag & BM_DIAG_PUBLISH) pub = BM_DIAG_PUBLISH;
+    // the groups run as parallel branches: the last work item of all of them finishes the step
+    for (auto &a : v) {
+        a.last_kind = lk;
+        a.diag |= pub;
+    }
     std::map<int, std::vector<StageArgs<T>>> groups;   // x length with a register kernel, or 0
     for (auto &a : v) groups[stage_reg_q(a.LX, 1) ? a.LX : 0].push_back(a);
-    size_t gi = 0;
+    const size_t first = c->bp.recs.size();
+    Branches br(c);
     for (auto &kv : groups) {
-        const bool last = (++gi == groups.size());
-        for (auto &a : kv.second) {
-            a.last_kind = last ? lk : BM_LAST_NONE;
-            a.diag = (a.diag & ~BM_DIAG_PUBLISH) | (last ? pub : 0);   // every block of the last launch counts
-        }
+        if (int rc = br.next()) return rc;
         if (int rc = stage_batch_one<T>(c, kv.first, kv.second, count)) return rc;
+    }
+    if (int rc = br.join()) return rc;
+    if (c->bp.collect) {
+        unsigned int total = 0;
+        for (size_t i = first; i < c->bp.recs.size(); i++) total += (unsigned int)c->bp.recs[i].nwork;
+        for (size_t i = first; i < c->bp.recs.size(); i++) c->bp.recs[i].total = total;
     }
     return 0;
 }
@@ -1424,18 +1510,30 @@ int yz_multi(bm_ctx *c, int gate, int *count)
         }
     }
     int rc;
-    for (auto &kv : g2)
-        if ((rc = yz_batch_one<T>(c, kv.first ? BM_BATCH_YMID2D_REG : BM_BATCH_YMID2D, kv.first, kv.second, count))) return rc;
     auto ykind = [](int key, bool inv) {
         return key > 0 ? (inv ? BM_BATCH_YINV_REG : BM_BATCH_YFWD_REG) : key < 0 ? (inv ? BM_BATCH_YINV_ST : BM_BATCH_YFWD_ST)
                                                                             : (inv ? BM_BATCH_YINV : BM_BATCH_YFWD);
     };
-    for (auto &kv : gy)
+    Branches br(c);
+    for (auto &kv : gy) {
+        if ((rc = br.next())) return rc;
         if ((rc = yz_batch_one<T>(c, ykind(kv.first, false), kv.first < 0 ? -kv.first : kv.first, kv.second, count))) return rc;
-    for (auto &kv : gz)
+    }
+    for (auto &kv : g2) {
+        if ((rc = br.next())) return rc;
+        if ((rc = yz_batch_one<T>(c, kv.first ? BM_BATCH_YMID2D_REG : BM_BATCH_YMID2D, kv.first, kv.second, count))) return rc;
+    }
+    if ((rc = br.join())) return rc;
+    for (auto &kv : gz) {
+        if ((rc = br.next())) return rc;
         if ((rc = yz_batch_one<T>(c, kv.first ? BM_BATCH_ZMID_REG : BM_BATCH_ZMID, kv.first, kv.second, count))) return rc;
-    for (auto &kv : gy)
+    }
+    if ((rc = br.join())) return rc;
+    for (auto &kv : gy) {
+        if ((rc = br.next())) return rc;
         if ((rc = yz_batch_one<T>(c, ykind(kv.first, true), kv.first < 0 ? -kv.first : kv.first, kv.second, count))) return rc;
+    }
+    if ((rc = br.join())) return rc;
     return 0;
 }
 
@@ -2028,6 +2126,8 @@ int build_graph(bm_ctx *c)
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(c->stream, &g);
         c->es_phase = 0;
+        for (auto ev : c->side_ev) cudaEventDestroy(ev);
+        c->side_ev.clear();
         if (rc) { if (g) cudaGraphDestroy(g); return rc; }
         if (e != cudaSuccess) return fail(BM_ECUDA, std::string("graph capture: ") + cudaGetErrorString(e));
         if (phase == 1) {
@@ -2365,6 +2465,7 @@ int bm_destroy(bm_ctx *c)
     for (auto &m : c->meshes) free_mesh(m);
     if (c->st) cudaFree(c->st);
     if (c->farq) cudaFree(c->farq);
+    for (auto st : c->side) cudaStreamDestroy(st);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
     return 0;

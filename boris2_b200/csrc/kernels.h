@@ -246,9 +246,10 @@ template <typename T> inline bool stage_adv_plain(const StageArgs<T> &a)
     return a.mode == BM_MODE_UPDATE && !a.staged && !a.es_fold && !a.Hd && !a.Hsave && !a.Ysave && a.copy_to && a.Mout &&
            a.do_xfwd && !a.ev_out && !a.renorm;
 }
+// total: work items of all the launches of the set, the last of which finishes the step
 // plain: every argument block of the launch satisfies stage_plain (FP32 takes the SPEC 1 kernels)
 template <typename T>
-int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem, cudaStream_t s,
+int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s,
                        int plain = 0);
 int stage_reg_q(int LX, int xv = 0);   // threads per x line of the register stage kernel, variant xv (0: generic kernel)
 int launch_scalar_reset(StepState *st, cudaStream_t s);

@@ -738,15 +738,15 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_stage(StageArgs<T> a)
 }
 
 // many meshes in one launch: work item (mesh, row block). The meshes share the step state; every
-// item takes part in the error-norm maximum and the last item finishes the step (last_kind is the
-// same for all meshes of the launch).
+// item takes part in the error-norm maximum, and the last of the `total` items of the set's launches
+// (which may run at the same time) finishes the step (last_kind is the same for all of them).
 template <typename T>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_stage_batch(const StageArgs<T> *__restrict__ args, const int2 *__restrict__ work,
-                                                                int nwork)
+                                                                int nwork, unsigned int total)
 {
     if (stage_gated_out<T>(args[0].st, args[0].gate) || (int)blockIdx.x >= nwork) return;
     const int2 it = work[blockIdx.x];
-    stage_generic_body<T>(args[it.x], it.y, (unsigned int)nwork);
+    stage_generic_body<T>(args[it.x], it.y, total);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1146,11 +1146,11 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX16_LO_MAXNREG_F) k_stage
 // block); the error-norm maximum and the step bookkeeping follow k_stage_batch
 template <typename T, int LX, int SPEC = 0>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx_batch(const StageArgs<T> *__restrict__ args,
-                                                                         const int2 *__restrict__ work, int nwork)
+                                                                         const int2 *__restrict__ work, int nwork, unsigned int total)
 {
     if (stage_gated_out<T>(args[0].st, args[0].gate) || (int)blockIdx.x >= nwork) return;
     const int2 it = work[blockIdx.x];
-    stage_reg_body<T, LX, 1, SPEC>(args[it.x], it.y, (unsigned int)nwork);
+    stage_reg_body<T, LX, 1, SPEC>(args[it.x], it.y, total);
 }
 
 template <typename T, int LX, int XV>
@@ -1240,15 +1240,15 @@ template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s)
 // radix-16 variant (x lengths 256 .. 1024)
 template <typename T, int LX, int SPEC = 0>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx16_batch(const StageArgs<T> *__restrict__ args,
-                                                                                       const int2 *__restrict__ work, int nwork)
+                                                                                       const int2 *__restrict__ work, int nwork, unsigned int total)
 {
     if (stage_gated_out<T>(args[0].st, args[0].gate) || (int)blockIdx.x >= nwork) return;
     const int2 it = work[blockIdx.x];
-    stage_reg_body<T, LX, 2, SPEC>(args[it.x], it.y, (unsigned int)nwork);
+    stage_reg_body<T, LX, 2, SPEC>(args[it.x], it.y, total);
 }
 
 template <typename T, int LX, int SPEC>
-static int launch_stage_rx_batch_s(const StageArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem, cudaStream_t s)
+static int launch_stage_rx_batch_s(const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s)
 {
     if constexpr (LX >= 256 && (LX % 3) != 0) {
         if (smem > BM_SMEM_DEFAULT_SAFE) {
@@ -1256,30 +1256,30 @@ static int launch_stage_rx_batch_s(const StageArgs<T> *dargs, const int2 *dwork,
                                                  BM_SMEM_CAP);
             if (e != cudaSuccess) return 2000 + (int)e;
         }
-        k_stage_rx16_batch<T, LX, SPEC><<<nwork, nt, smem, s>>>(dargs, dwork, nwork);
+        k_stage_rx16_batch<T, LX, SPEC><<<nwork, nt, smem, s>>>(dargs, dwork, nwork, total);
         return (int)cudaGetLastError();
     }
     if (smem > BM_SMEM_DEFAULT_SAFE) {
         cudaError_t e = cudaFuncSetAttribute(k_stage_rx_batch<T, LX, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, BM_SMEM_CAP);
         if (e != cudaSuccess) return (int)e;
     }
-    k_stage_rx_batch<T, LX, SPEC><<<nwork, nt, smem, s>>>(dargs, dwork, nwork);
+    k_stage_rx_batch<T, LX, SPEC><<<nwork, nt, smem, s>>>(dargs, dwork, nwork, total);
     return (int)cudaGetLastError();
 }
 
 // the plain-stage instantiation for FP32 launches whose argument blocks are all plain (stage_plain)
 template <typename T, int LX>
-static int launch_stage_rx_batch(const StageArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem, cudaStream_t s,
+static int launch_stage_rx_batch(const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s,
                                  int plain)
 {
     if constexpr (sizeof(T) == 4) {
-        if (plain) return launch_stage_rx_batch_s<T, LX, 1>(dargs, dwork, nwork, nt, smem, s);
+        if (plain) return launch_stage_rx_batch_s<T, LX, 1>(dargs, dwork, nwork, total, nt, smem, s);
     }
-    return launch_stage_rx_batch_s<T, LX, 0>(dargs, dwork, nwork, nt, smem, s);
+    return launch_stage_rx_batch_s<T, LX, 0>(dargs, dwork, nwork, total, nt, smem, s);
 }
 
 template <typename T>
-int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem, cudaStream_t s,
+int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s,
                        int plain)
 {
     if (nwork < 1) return 0;
@@ -1287,26 +1287,26 @@ int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, in
     if (smem > 200 * 1024) return 212;
     switch (key) {
     case 0: break;
-    case 16: return launch_stage_rx_batch<T, 16>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 32: return launch_stage_rx_batch<T, 32>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 64: return launch_stage_rx_batch<T, 64>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 128: return launch_stage_rx_batch<T, 128>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 256: return launch_stage_rx_batch<T, 256>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 512: return launch_stage_rx_batch<T, 512>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 1024: return launch_stage_rx_batch<T, 1024>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 24: return launch_stage_rx_batch<T, 24>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 48: return launch_stage_rx_batch<T, 48>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 96: return launch_stage_rx_batch<T, 96>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 192: return launch_stage_rx_batch<T, 192>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 384: return launch_stage_rx_batch<T, 384>(dargs, dwork, nwork, nt, smem, s, plain);
-    case 768: return launch_stage_rx_batch<T, 768>(dargs, dwork, nwork, nt, smem, s, plain);
+    case 16: return launch_stage_rx_batch<T, 16>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 32: return launch_stage_rx_batch<T, 32>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 64: return launch_stage_rx_batch<T, 64>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 128: return launch_stage_rx_batch<T, 128>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 256: return launch_stage_rx_batch<T, 256>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 512: return launch_stage_rx_batch<T, 512>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 1024: return launch_stage_rx_batch<T, 1024>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 24: return launch_stage_rx_batch<T, 24>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 48: return launch_stage_rx_batch<T, 48>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 96: return launch_stage_rx_batch<T, 96>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 192: return launch_stage_rx_batch<T, 192>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 384: return launch_stage_rx_batch<T, 384>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 768: return launch_stage_rx_batch<T, 768>(dargs, dwork, nwork, total, nt, smem, s, plain);
     default: return 213;
     }
     if (smem > BM_SMEM_DEFAULT_SAFE) {
         cudaError_t e = cudaFuncSetAttribute(k_stage_batch<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, BM_SMEM_CAP);
         if (e != cudaSuccess) return (int)e;
     }
-    k_stage_batch<T><<<nwork, nt, smem, s>>>(dargs, dwork, nwork);
+    k_stage_batch<T><<<nwork, nt, smem, s>>>(dargs, dwork, nwork, total);
     return (int)cudaGetLastError();
 }
 
