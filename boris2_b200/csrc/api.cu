@@ -124,7 +124,7 @@ struct BatchRec {
     int nwork, nt;
     unsigned int total = 0;   // stage launches: work items of the set's launches together
     size_t smem;
-    int plain = 0;        // stage launch: every argument block is a plain stage update (stage_plain)
+    int kind_s = 0;       // stage launch: bit 0 every argument block is a plain stage update, bit 1 some nx is odd
 };
 struct BatchPlan {
     bool collect = false;
@@ -1329,8 +1329,9 @@ int stage_batch_one(bm_ctx *c, int key, std::vector<StageArgs<T>> &v, int *count
         r.nwork = (int)work.size();
         r.nt = nt;
         r.smem = smem;
-        r.plain = key ? 1 : 0;
-        for (auto &a : v) if (!stage_plain(a)) r.plain = 0;
+        r.kind_s = key ? 1 : 0;
+        for (auto &a : v) if (!stage_plain(a)) r.kind_s &= ~1;
+        for (auto &a : v) if (a.nx & 1) r.kind_s |= 2;
         bp.recs.push_back(r);
         return 0;
     }
@@ -1338,7 +1339,7 @@ int stage_batch_one(bm_ctx *c, int key, std::vector<StageArgs<T>> &v, int *count
     const BatchRec &r = bp.recs[bp.next++];
     const char *base = (const char *)bp.dbuf;
     CKL(launch_stage_batch<T>(r.key, (const StageArgs<T> *)(base + r.args_off), (const int2 *)(base + r.work_off), r.nwork,
-                              r.total, r.nt, r.smem, c->stream, r.plain), "stage batch");
+                              r.total, r.nt, r.smem, c->stream, r.kind_s), "stage batch");
     (*count)++;
     return 0;
 }

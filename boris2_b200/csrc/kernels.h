@@ -247,10 +247,10 @@ template <typename T> inline bool stage_adv_plain(const StageArgs<T> &a)
            a.do_xfwd && !a.ev_out && !a.renorm;
 }
 // total: work items of all the launches of the set, the last of which finishes the step
-// plain: every argument block of the launch satisfies stage_plain (FP32 takes the SPEC 1 kernels)
+// kind: bit 0 every argument block satisfies stage_plain (FP32 takes the SPEC 1 kernels), bit 1 some nx is odd
 template <typename T>
 int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s,
-                       int plain = 0);
+                       int kind = 0);
 int stage_reg_q(int LX, int xv = 0);   // threads per x line of the register stage kernel, variant xv (0: generic kernel)
 int launch_scalar_reset(StepState *st, cudaStream_t s);
 

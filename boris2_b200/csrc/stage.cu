@@ -1,6 +1,14 @@
-// x-length queries of the stage kernel (stage.cuh) and its FP32 instantiations; FP64 and the batched
-// launches are translation units of their own, so that they compile in parallel.
+// x-length queries of the stage kernel (stage.cuh) and its launcher; the register kernels of each variant
+// and precision and the batched launches are translation units of their own, so that they compile in parallel.
 #include "stage.cuh"
+
+extern template int launch_stage_variant<float, 0>(const StageArgs<float> &, cudaStream_t);
+extern template int launch_stage_variant<float, 1>(const StageArgs<float> &, cudaStream_t);
+extern template int launch_stage_variant<float, 2>(const StageArgs<float> &, cudaStream_t);
+extern template int launch_stage_variant<float, 3>(const StageArgs<float> &, cudaStream_t);
+extern template int launch_stage_variant<double, 0>(const StageArgs<double> &, cudaStream_t);
+extern template int launch_stage_variant<double, 1>(const StageArgs<double> &, cudaStream_t);
+extern template int launch_stage_variant<double, 2>(const StageArgs<double> &, cudaStream_t);
 
 // x lengths with a register kernel and their threads per line
 int stage_reg_q(int LX, int xv)
@@ -30,3 +38,4 @@ bool stage_reg_path(int LX, int xv)
 }
 
 template int launch_stage<float>(const StageArgs<float> &, cudaStream_t);
+template int launch_stage<double>(const StageArgs<double> &, cudaStream_t);

@@ -156,26 +156,8 @@ __device__ __forceinline__ void axis_stencil(const T m[3], const T *mp, const T 
 // Per-cell part of a stage: Heff, LLG, update. `lines` holds the 3 * rpb packed x lines of the
 // block (component-major), element e of line q at sm[q * LSP + addr(e)]; on entry it carries
 // the unscaled inverse-x result (H_demag / scale), on exit the new M (when do_xfwd).
-// Per-cell input accessors. AccGlobal reads the device arrays; AccStaged reads the rows the
-// register kernel prefetched into shared memory (layout: stage_layout in kernels.h).
-template <typename T> struct AccGlobal {
-    // pointers copied out of the argument block so each access is (per-cell base)[uniform offset]
-    const T *Mn, *Mb, *E[6], *Msm, *K1m;
-    long long n, off[5];
-    __device__ AccGlobal(const StageArgs<T> &aa) : Mn(aa.Min), Mb(aa.Mbase), Msm(aa.Ms_map), K1m(aa.K1_map), n(aa.n)
-    {
-#pragma unroll
-        for (int i = 0; i < 6; i++) E[i] = aa.ev[i];
-        long long nxy = (long long)aa.nx * aa.ny;
-        off[0] = 0; off[1] = -aa.nx; off[2] = aa.nx; off[3] = -nxy; off[4] = nxy;
-    }
-    __device__ __forceinline__ T m(int, int slot, int c, int, long long cell) const { return (Mn + cell)[c * n + off[slot]]; }
-    __device__ __forceinline__ T mb(int, int c, int, long long cell) const { return (Mb + cell)[c * n]; }
-    __device__ __forceinline__ T ev(int i, int, int c, int, long long cell) const { return (E[i] + cell)[c * n]; }
-    __device__ __forceinline__ T ms(int, int, long long cell) const { return Msm[cell]; }
-    __device__ __forceinline__ T k1(int, int, long long cell) const { return K1m[cell]; }
-};
-
+// Per-cell input accessor of the rows the register kernel prefetched into shared memory (layout:
+// stage_layout in kernels.h).
 template <typename T> struct AccStaged {
     const T *R;
     int nx, kr, ns3, hasmb, evo, mso, k1o;
@@ -242,28 +224,20 @@ template <typename T> __device__ __forceinline__ int stage_diag_active(const Sta
     return d;
 }
 
-// SPEC 1: the plain stage update (stage_plain on the host): mode, the outputs written and the demag
-// and exchange terms are compile-time, so their run-time checks leave the per-cell loop; SPEC 2 the
-// plain RKDP54 error estimate (stage_lte_plain), SPEC 3 the plain advance of the base state
-// (stage_adv_plain), likewise
-template <typename T, int SPEC = 0, typename AddrF, typename Acc>
+template <typename T, typename AddrF, typename Acc>
 __device__ __forceinline__ void stage_cells(const StageArgs<T> &a, cpx<T> *sm, int LSP, AddrF addr, int r0, double &lmax,
                                             const Acc &acc)
 {
-    constexpr bool PS = SPEC == 1, PL = SPEC == 2, PA = SPEC == 3, SP = SPEC != 0;
     const int nx = a.nx, ny = a.ny, nz = a.nz, rpb = a.rpb;
     const int nrows = ny * nz;
     const int tid = threadIdx.x, nt = blockDim.x;
     const long long n = a.n;
-    const int mode = PS ? BM_MODE_STAGE : PL ? BM_MODE_LTE : PA ? BM_MODE_UPDATE : a.mode;
-    const T *Hd = SP ? nullptr : a.Hd;
-    T *Hsave = SP ? nullptr : a.Hsave;
-    T *Ysave = SP ? nullptr : a.Ysave;
-    T *copy_to = (PS || PL) ? nullptr : a.copy_to;
-    const bool has_ev_out = (PS || PL) || (!PA && a.ev_out), has_Mout = (PS || PA) || (!PL && a.Mout);
-    const bool do_xfwd = (PS || PA) || (!PL && a.do_xfwd);
-    const bool fields = (PS || PL) || (!PA && mode != BM_MODE_UPDATE);
-    const bool demag = (PS || PL) || (!PA && fields && (a.modules & BM_MOD_DEMAG));
+    const int mode = a.mode;
+    const T *Hd = a.Hd;
+    T *Hsave = a.Hsave, *Ysave = a.Ysave, *copy_to = a.copy_to;
+    const bool has_ev_out = a.ev_out, has_Mout = a.Mout, do_xfwd = a.do_xfwd;
+    const bool fields = mode != BM_MODE_UPDATE;
+    const bool demag = fields && (a.modules & BM_MOD_DEMAG);
     const double dT = a.st ? *((volatile double *)&a.st->dT) : 0.0;
     T Ha[3] = {0, 0, 0};
     if (fields && (a.modules & BM_MOD_ZEEMAN) && a.Ha && a.nHa > 0) {
@@ -279,7 +253,7 @@ __device__ __forceinline__ void stage_cells(const StageArgs<T> &a, cpx<T> *sm, i
         }
         Ha[0] = (T)a.Ha[3 * hi]; Ha[1] = (T)a.Ha[3 * hi + 1]; Ha[2] = (T)a.Ha[3 * hi + 2];
     }
-    const bool exch = (PS || PL) || (!PA && fields && (a.modules & (BM_MOD_EXCH | BM_MOD_IDMI)));
+    const bool exch = fields && (a.modules & (BM_MOD_EXCH | BM_MOD_IDMI));
     const bool idmi = (a.modules & BM_MOD_IDMI) != 0;
     const bool zflat = (nz == 1);
     // torque / dm/dt diagnostics of this launch (meshes with grel = 0 take no part, as in the
@@ -519,7 +493,7 @@ __device__ __forceinline__ void stage_cells(const StageArgs<T> &a, cpx<T> *sm, i
 #pragma unroll
             for (int c = 0; c < 3; c++) (Ysave + cell)[c * n] = mn[c];
         }
-        if (!PA && a.renorm) {
+        if (a.renorm) {
             T f = Ms / sqrt(mn[0] * mn[0] + mn[1] * mn[1] + mn[2] * mn[2]);
             mn[0] *= f; mn[1] *= f; mn[2] *= f;
             // the step's new state must be finite (the sum is non-finite if any component is)
@@ -566,6 +540,8 @@ __device__ __forceinline__ void stage_cells(const StageArgs<T> &a, cpx<T> *sm, i
         cell_body(r, x, y, z, (long long)row * nx + x);
     }
 }
+
+#include "stage_pairs.cuh"
 
 // LTE block reduction and the last-block bookkeeping (step finish / controller / restore flag)
 // total: launch items that each call the tail once (blocks, or work items of a batched launch)
@@ -712,7 +688,8 @@ __device__ __forceinline__ void stage_generic_body(const StageArgs<T> &a, int bi
         fft_line<T, true, true>(line, 1, t, qact, a.px, a.twx);
     }
     double lmax = 0.0;
-    stage_cells<T>(a, sm, LSP, [](int e) { return eaddr<true>(e, 1); }, r0, lmax, AccGlobal<T>(a));
+    if (a.nx & 1) stage_pairs<T, 0, true>(a, sm, LSP, [](int e) { return eaddr<true>(e, 1); }, r0, lmax);
+    else stage_pairs<T, 0, false>(a, sm, LSP, [](int e) { return eaddr<true>(e, 1); }, r0, lmax);
     if (a.do_xfwd) {
         const int first_pad = (a.nx + 1) >> 1;
         for (int idx = tid; idx < 3 * rpb * LX; idx += blockDim.x) {
@@ -983,9 +960,13 @@ __device__ __forceinline__ void stage_prefetch_rows(const StageArgs<T> &a, int r
     }
 }
 
-template <typename T, int LX, int XV, int SPEC = 0>
+// Instantiations of the register stage kernels (KS): 0 .. 3 the pair form at SPEC 0 .. 3 for even nx, 4 the
+// one-cell form on staged rows, 5 and 6 the pair form at SPEC 0 and 1 for any nx.
+template <typename T, int LX, int XV, int KS = 0>
 __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, unsigned int total)
 {
+    constexpr int SPEC = KS == 6 ? 1 : KS >= 4 ? 0 : KS;
+    constexpr bool ODD = KS >= 5, STAGED = KS == 4;
     extern __shared__ unsigned char smraw[];
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
     using C = xr_cfg<LX, XV>;
@@ -1010,10 +991,10 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
     cp_async_commit();
     // without staging: L2 prefetch of the rows the per-cell phase reads from DRAM, so that they arrive
     // while the inverse transform runs
-    if (!a.staged && (a.mode != BM_MODE_UPDATE || a.Mbase != a.Min)) stage_prefetch_rows<T>(a, r0);
+    if (!STAGED && (a.mode != BM_MODE_UPDATE || a.Mbase != a.Min)) stage_prefetch_rows<T>(a, r0);
     // group 2: the per-cell input rows, arriving while the inverse transform runs
     AccStaged<T> st;
-    if (a.staged) {
+    if constexpr (STAGED) {
         const StageLayout L = stage_layout(a);
         const int nx = a.nx, ny = a.ny, nz = a.nz;
         const long long n = a.n;
@@ -1081,8 +1062,8 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
     cp_async_wait_group<0>();
     __syncthreads();
     double lmax = 0.0;
-    if (SPEC == 0 && a.staged) stage_cells<T>(a, sm, LSP, A, r0, lmax, st);
-    else stage_cells<T, SPEC>(a, sm, LSP, A, r0, lmax, AccGlobal<T>(a));
+    if constexpr (STAGED) stage_cells<T>(a, sm, LSP, A, r0, lmax, st);
+    else stage_pairs<T, SPEC, ODD>(a, sm, LSP, A, r0, lmax);
     if (SPEC == 1 || SPEC == 3 || (SPEC == 0 && a.do_xfwd)) {
         for (int idx = tid; idx < 3 * rpb * (LX / 2); idx += blockDim.x) {
             int qq = idx / (LX / 2), mm = idx - qq * (LX / 2);
@@ -1113,18 +1094,18 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
     stage_tail<T, SPEC>(a, lmax, total);
 }
 
-template <typename T, int LX>
+template <typename T, int LX, int KS>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_stage_reg(StageArgs<T> a)
 {
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_reg_body<T, LX, 0>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<T, LX, 0, KS>(a, blockIdx.x, gridDim.x);
 }
 
-template <typename T, int LX>
+template <typename T, int LX, int KS>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx(StageArgs<T> a)
 {
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_reg_body<T, LX, 1>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<T, LX, 1, KS>(a, blockIdx.x, gridDim.x);
 }
 
 template <typename T, int LX, int SPEC>
@@ -1169,18 +1150,23 @@ static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
         if (lb + rb <= 200 * 1024) smem = lb + rb;
         else b.staged = 0;
     }
+    // the instantiation (KS): the two-level kernel has the general ones, the radix-8 kernel the plain stage
+    // update too, the radix-16 kernels all
+    const bool odd = b.nx & 1;
+    const int sp = stage_plain(b) ? 1 : stage_lte_plain(b) ? 2 : stage_adv_plain(b) ? 3 : 0;
     void (*kern)(StageArgs<T>);
-    if constexpr (XV == 0) kern = k_stage_reg<T, LX>;
-    else if constexpr (XV == 1) kern = k_stage_rx<T, LX>;
-    else {
-        const int sp = stage_plain(b) ? 1 : stage_lte_plain(b) ? 2 : stage_adv_plain(b) ? 3 : 0;
-        if constexpr (XV == 2)
-            kern = sp == 1 ? k_stage_rx16<T, LX, 1> : sp == 2 ? k_stage_rx16<T, LX, 2> : sp == 3 ? k_stage_rx16<T, LX, 3>
-                                                                                          : k_stage_rx16<T, LX, 0>;
-        else
-            kern = sp == 1 ? k_stage_rx16_lo<T, LX, 1> : sp == 2 ? k_stage_rx16_lo<T, LX, 2>
-                         : sp == 3 ? k_stage_rx16_lo<T, LX, 3> : k_stage_rx16_lo<T, LX, 0>;
-    }
+    if constexpr (XV == 0) kern = b.staged ? k_stage_reg<T, LX, 4> : odd ? k_stage_reg<T, LX, 5> : k_stage_reg<T, LX, 0>;
+    else if constexpr (XV == 1)
+        kern = b.staged ? k_stage_rx<T, LX, 4> : odd ? (sp == 1 ? k_stage_rx<T, LX, 6> : k_stage_rx<T, LX, 5>)
+                                               : (sp == 1 ? k_stage_rx<T, LX, 1> : k_stage_rx<T, LX, 0>);
+    else if constexpr (XV == 2)
+        kern = b.staged ? k_stage_rx16<T, LX, 4> : odd ? (sp == 1 ? k_stage_rx16<T, LX, 6> : k_stage_rx16<T, LX, 5>)
+             : sp == 1 ? k_stage_rx16<T, LX, 1> : sp == 2 ? k_stage_rx16<T, LX, 2> : sp == 3 ? k_stage_rx16<T, LX, 3>
+                                                                                   : k_stage_rx16<T, LX, 0>;
+    else
+        kern = b.staged ? k_stage_rx16_lo<T, LX, 4> : odd ? (sp == 1 ? k_stage_rx16_lo<T, LX, 6> : k_stage_rx16_lo<T, LX, 5>)
+             : sp == 1 ? k_stage_rx16_lo<T, LX, 1> : sp == 2 ? k_stage_rx16_lo<T, LX, 2> : sp == 3 ? k_stage_rx16_lo<T, LX, 3>
+                                                                                      : k_stage_rx16_lo<T, LX, 0>;
     if (smem > BM_SMEM_DEFAULT_SAFE) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BM_SMEM_CAP);
         if (e != cudaSuccess) return 2000 + (int)e;   // the shared-memory ceiling was refused
@@ -1191,37 +1177,49 @@ static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
     return (int)cudaGetLastError();
 }
 
-template <typename T, int LX> static int launch_stage_xv(const StageArgs<T> &a, cudaStream_t s)
+// the register stage kernels of one x-transform variant; -1: the variant has none of this length
+template <typename T, int XV> int launch_stage_variant(const StageArgs<T> &a, cudaStream_t s)
 {
-    if constexpr (LX >= 256) {
-        // xv 3 is its own kernel for FP32 only (the FP64 cap is the same for both)
-        if constexpr (sizeof(T) == 4) {
-            if (a.xv == 3) return launch_stage_reg<T, LX, 3>(a, s);
+    if constexpr (XV <= 1) {
+        switch (a.LX) {
+        case 16: return launch_stage_reg<T, 16, XV>(a, s);
+        case 32: return launch_stage_reg<T, 32, XV>(a, s);
+        case 64: return launch_stage_reg<T, 64, XV>(a, s);
+        case 128: return launch_stage_reg<T, 128, XV>(a, s);
+        default: break;
         }
-        if (a.xv == 2 || a.xv == 3) return launch_stage_reg<T, LX, 2>(a, s);
     }
-    return a.xv ? launch_stage_reg<T, LX, 1>(a, s) : launch_stage_reg<T, LX, 0>(a, s);
+    if constexpr (XV == 1) {
+        switch (a.LX) {
+        case 24: return launch_stage_reg<T, 24, 1>(a, s);
+        case 48: return launch_stage_reg<T, 48, 1>(a, s);
+        case 96: return launch_stage_reg<T, 96, 1>(a, s);
+        case 192: return launch_stage_reg<T, 192, 1>(a, s);
+        case 384: return launch_stage_reg<T, 384, 1>(a, s);
+        case 768: return launch_stage_reg<T, 768, 1>(a, s);
+        default: break;
+        }
+    }
+    switch (a.LX) {
+    case 256: return launch_stage_reg<T, 256, XV>(a, s);
+    case 512: return launch_stage_reg<T, 512, XV>(a, s);
+    case 1024: return launch_stage_reg<T, 1024, XV>(a, s);
+    default: return -1;
+    }
 }
-
 
 template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s)
 {
-    switch (a.LX) {
-    case 16: return launch_stage_xv<T, 16>(a, s);
-    case 32: return launch_stage_xv<T, 32>(a, s);
-    case 64: return launch_stage_xv<T, 64>(a, s);
-    case 128: return launch_stage_xv<T, 128>(a, s);
-    case 256: return launch_stage_xv<T, 256>(a, s);
-    case 512: return launch_stage_xv<T, 512>(a, s);
-    case 1024: return launch_stage_xv<T, 1024>(a, s);
-    case 24: if (a.xv) return launch_stage_reg<T, 24, 1>(a, s); break;
-    case 48: if (a.xv) return launch_stage_reg<T, 48, 1>(a, s); break;
-    case 96: if (a.xv) return launch_stage_reg<T, 96, 1>(a, s); break;
-    case 192: if (a.xv) return launch_stage_reg<T, 192, 1>(a, s); break;
-    case 384: if (a.xv) return launch_stage_reg<T, 384, 1>(a, s); break;
-    case 768: if (a.xv) return launch_stage_reg<T, 768, 1>(a, s); break;
-    default: break;
+    int rc = -1;
+    if (a.LX >= 256 && a.LX % 3) {
+        // xv 3 is its own kernel for FP32 only (the FP64 cap is the same for both)
+        if constexpr (sizeof(T) == 4) {
+            if (a.xv == 3) rc = launch_stage_variant<T, 3>(a, s);
+        }
+        if (rc < 0 && a.xv >= 2) rc = launch_stage_variant<T, 2>(a, s);
     }
+    if (rc < 0) rc = a.xv ? launch_stage_variant<T, 1>(a, s) : launch_stage_variant<T, 0>(a, s);
+    if (rc >= 0) return rc;
     int nt = (3 * a.rpb * a.px.tpl + 31) & ~31;   // whole warps
     if (nt > bm_lb<T>::v) return 201;
     size_t smem = (size_t)3 * a.rpb * padded_len(a.LX) * sizeof(cpx<T>);
@@ -1267,39 +1265,41 @@ static int launch_stage_rx_batch_s(const StageArgs<T> *dargs, const int2 *dwork,
     return (int)cudaGetLastError();
 }
 
-// the plain-stage instantiation for FP32 launches whose argument blocks are all plain (stage_plain)
+// kind: bit 0 every argument block is a plain stage update (FP32 has that instantiation), bit 1 some nx is odd
 template <typename T, int LX>
 static int launch_stage_rx_batch(const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s,
-                                 int plain)
+                                 int kind)
 {
     if constexpr (sizeof(T) == 4) {
-        if (plain) return launch_stage_rx_batch_s<T, LX, 1>(dargs, dwork, nwork, total, nt, smem, s);
+        if ((kind & 1) && (kind & 2)) return launch_stage_rx_batch_s<T, LX, 6>(dargs, dwork, nwork, total, nt, smem, s);
+        if (kind & 1) return launch_stage_rx_batch_s<T, LX, 1>(dargs, dwork, nwork, total, nt, smem, s);
     }
+    if (kind & 2) return launch_stage_rx_batch_s<T, LX, 5>(dargs, dwork, nwork, total, nt, smem, s);
     return launch_stage_rx_batch_s<T, LX, 0>(dargs, dwork, nwork, total, nt, smem, s);
 }
 
 template <typename T>
 int launch_stage_batch(int key, const StageArgs<T> *dargs, const int2 *dwork, int nwork, unsigned int total, int nt, size_t smem, cudaStream_t s,
-                       int plain)
+                       int kind)
 {
     if (nwork < 1) return 0;
     if (nt > bm_lb<T>::v || nt < 32) return 211;
     if (smem > 200 * 1024) return 212;
     switch (key) {
     case 0: break;
-    case 16: return launch_stage_rx_batch<T, 16>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 32: return launch_stage_rx_batch<T, 32>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 64: return launch_stage_rx_batch<T, 64>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 128: return launch_stage_rx_batch<T, 128>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 256: return launch_stage_rx_batch<T, 256>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 512: return launch_stage_rx_batch<T, 512>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 1024: return launch_stage_rx_batch<T, 1024>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 24: return launch_stage_rx_batch<T, 24>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 48: return launch_stage_rx_batch<T, 48>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 96: return launch_stage_rx_batch<T, 96>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 192: return launch_stage_rx_batch<T, 192>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 384: return launch_stage_rx_batch<T, 384>(dargs, dwork, nwork, total, nt, smem, s, plain);
-    case 768: return launch_stage_rx_batch<T, 768>(dargs, dwork, nwork, total, nt, smem, s, plain);
+    case 16: return launch_stage_rx_batch<T, 16>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 32: return launch_stage_rx_batch<T, 32>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 64: return launch_stage_rx_batch<T, 64>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 128: return launch_stage_rx_batch<T, 128>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 256: return launch_stage_rx_batch<T, 256>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 512: return launch_stage_rx_batch<T, 512>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 1024: return launch_stage_rx_batch<T, 1024>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 24: return launch_stage_rx_batch<T, 24>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 48: return launch_stage_rx_batch<T, 48>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 96: return launch_stage_rx_batch<T, 96>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 192: return launch_stage_rx_batch<T, 192>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 384: return launch_stage_rx_batch<T, 384>(dargs, dwork, nwork, total, nt, smem, s, kind);
+    case 768: return launch_stage_rx_batch<T, 768>(dargs, dwork, nwork, total, nt, smem, s, kind);
     default: return 213;
     }
     if (smem > BM_SMEM_DEFAULT_SAFE) {

@@ -1,0 +1,4 @@
+// Register stage kernels of x-transform variant 0, FP32 (stage.cuh)
+#include "stage.cuh"
+
+template int launch_stage_variant<float, 0>(const StageArgs<float> &, cudaStream_t);

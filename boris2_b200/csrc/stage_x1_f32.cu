@@ -1,0 +1,4 @@
+// Register stage kernels of x-transform variant 1, FP32 (stage.cuh)
+#include "stage.cuh"
+
+template int launch_stage_variant<float, 1>(const StageArgs<float> &, cudaStream_t);

@@ -1,0 +1,39 @@
+"""Kernels that carry two x-adjacent values per thread, on cuda:0 against the oracle: the stage kernel's
+per-cell part on cell pairs (even and odd nx down to 1, every field term, open and periodic, each x
+transform variant).
+Bounds as elsewhere: FP64 1e-9 and mixed 1e-5 of the largest field, states FP64 1e-9, mixed 1e-4 of Ms."""
+import numpy as np
+import pytest
+
+from oracle_libs import sphere_random, OracleSolver
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nx", [1, 2, 3, 16, 31, 190, 257])
+@pytest.mark.parametrize("pbc", [(0, 0, 0), (2, -1, 1)])
+@pytest.mark.parametrize("xv", ["0", "1", "2"])
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-9), ("mixed", 1e-4)])
+def test_stage_pairs(bm, monkeypatch, nx, pbc, xv, prec, tol):
+    monkeypatch.setenv("BM_TILES", "1,1,4,2")
+    monkeypatch.setenv("BM_STAGE_XV", xv)
+    d = dict(n=(nx, 5, 3), h=(4e-9, 3e-9, 2e-9), Ms=8e5, A=1.3e-11, D=1.5e-3, alpha=0.1, K1=1e5, K2=2e4, ea=(0.3, 0.2, 0.9),
+             modules=1 | 4 | 8 | 16, Ha=(2e4, -1e4, 5e3), pbc=pbc)
+    M = sphere_random(int(np.prod(d["n"])), seed=9 + nx, Ms=8e5)
+    for ode in (0, 1):
+        s = OracleSolver([d], evaluation=ode, dt=2e-14)
+        s.set_m(M)
+        with bm.Context(precision=bm.FP64 if prec == "fp64" else bm.MIXED) as c:
+            c.add_mesh(d["n"], d["h"])
+            c.set_material(0, Ms=d["Ms"], A=d["A"], alpha=d["alpha"], K1=d["K1"], K2=d["K2"], ea=d["ea"], D=d["D"])
+            c.set_modules(0, d["modules"])
+            c.set_pbc(0, pbc)
+            c.set_field(0, d["Ha"])
+            c.setode("RKDP54" if ode else "RK4", 2e-14)
+            c.set_m(M)
+            H, Href = c.update_field(), s.heff()
+            assert np.abs(H - Href).max() / np.abs(Href).max() < (1e-9 if prec == "fp64" else 1e-5)
+            c.run(6)
+            s.run(6)
+            assert np.abs(c.get_m() - s.get_m()).max() / 8e5 < tol
+        s.close()
