@@ -194,6 +194,7 @@ struct bm_ctx {
     long long es_max_plane = 0;
     bool es_reset = true;       // clear the saved fields at the next state upload
     LaunchTimer *lt = nullptr;  // set while bm_time_step enqueues its eager steps
+    bool pdl = false;           // launches of a single field evaluation outside a graph (PdlScope)
     size_t mem_limit = 0;       // bm_set_memory_limit (0: the free device memory is the limit)
 };
 
@@ -1196,6 +1197,7 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     a.S1 = (cpx<T> *)m.S1;
     a.twx = (const cpx<T> *)m.twx; a.twx2 = (const cpx<T> *)m.twx2;
     a.px = m.px;
+    a.pdl = c->pdl;
     a.rpb = m.rpb;
     a.scale = (T)(2.0 / ((double)m.Nx * m.Ny * m.Nz));
     a.modules = m.modules;
@@ -1251,6 +1253,7 @@ struct Branches {
             if (!(fork = event())) return fail(BM_ECUDA, "branch event");
             CK(cudaEventRecord(fork, main));
             return 0;
+    a.pdl = c->pdl;
         }
         const int k = turn++ % kSide;
         while ((int)c->side.size() <= k) {
@@ -2233,9 +2236,20 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
 // ------------------------------------------------------------------ discrete adjoint of RK4
 // Forward: the step graph with a checkpoint of M and the time every k steps. Backward, per segment
 // from the last: restore the checkpoint, replay a captured graph that recomputes the segment's k
+// Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
+// latency between them (demag field of 32 x 16 x 1 cells 32 -> 28 us, of 200 x 150 x 12 in FP64 201 -> 191).
+// The captured steps don't take it: graph edges are as short already, and the next kernel's early blocks
+// cost the last wave of the one before (512 x 512 x 16 film, four RKDP54 steps 12.9 -> 13.4 ms).
+struct PdlScope {
+    bm_ctx *c;
+    explicit PdlScope(bm_ctx *ctx) : c(ctx) { c->pdl = true; }
+    ~PdlScope() { c->pdl = false; }
+};
+
 // steps with the fused stage kernels also writing each stage's input, field and pre-normalisation
 // update into a k-slot cache, then replay a captured graph that walks the k steps in reverse
 // (renormalisation VJP, then per stage the LLG / local-field VJP, the demag of gH through the
+    PdlScope pdl(c);
 // convolution pipeline, and the Laplacian / accumulation kernel). Gradients accumulate in FP64;
 // the Zeeman gradient of each step is summed per step and mapped to its sample on the host with
 // the step start time the device used.
@@ -2907,6 +2921,7 @@ int get_m_device_T(bm_ctx *c, Mesh &m, void *M, int eb)
     else CKL((launch_planes_to_daos<double, T>((double *)M, B<T>(m, 0), m.n, 0, nullptr, nullptr, c->stream)), "M out");
     CK(cudaStreamSynchronize(c->stream));
     return 0;
+    PdlScope pdl(c);
 }
 
 int device_entry_checks(bm_ctx *c, int mesh, const void *p, int eb, void *stream)

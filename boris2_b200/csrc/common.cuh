@@ -49,6 +49,37 @@ __device__ __forceinline__ void cp_async_real(T *smem, const T *gmem, bool valid
 }
 #endif
 
+#ifdef __CUDACC__
+// Programmatic dependent launch. Kernels that may be launched with the attribute (launch_pdl, pdl != 0) begin
+// with pdl_enter(): their blocks may become resident while the last blocks of the kernel before are still
+// running (launch_dependents) and wait there until that kernel has completed and its writes are visible (wait;
+// nothing to wait for after an ordinary launch). Every block of such a kernel passes the wait, so a completed
+// kernel implies that all kernels before it have completed.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_enter()
+{
+    pdl_trigger();
+    pdl_wait();
+}
+template <typename A>
+inline int launch_pdl(void (*kern)(A), dim3 grid, int nt, size_t smem, cudaStream_t s, const A &a, int pdl)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)nt);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, a);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+#endif
+
 // Physical constants (the reference's BorisLib/Funcs_Math_base.h:9,16)
 #define BM_MU0 1.256637061435916e-6
 #define BM_GAMMA 2.212761569e5

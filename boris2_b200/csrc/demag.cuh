@@ -130,6 +130,7 @@ __device__ __forceinline__ void ymid2d_body(const YZArgs<T> &a, int bx)
 template <typename T>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_ymid2d(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     ymid2d_body<T>(a, blockIdx.x);
 }
@@ -182,6 +183,7 @@ __device__ __forceinline__ void ypass3d_body(const YZArgs<T> &a, int bx, int z, 
 template <typename T, bool INV>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_ypass3d(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     ypass3d_body<T, INV>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -310,6 +312,7 @@ __device__ __forceinline__ void zmid_body(const YZArgs<T> &a, int bx, int ky)
 template <typename T>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_zmid(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     zmid_body<T>(a, blockIdx.x, blockIdx.y);
 }
@@ -466,6 +469,7 @@ __device__ __forceinline__ void pf_segment(const void *p0, const void *p1)
 template <typename T, int NZ, int WC>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_zmid_reg(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     zmid_reg_body<T, NZ, WC>(a, blockIdx.x, blockIdx.y);
 }
@@ -494,8 +498,7 @@ static int launch_zmid_reg_w(const YZArgs<T> &a, cudaStream_t s)
         if (e != cudaSuccess) return (int)e;
     }
     dim3 grid((a.LX + a.W - 1) / a.W, a.Ny / 2 + 1);
-    k_zmid_reg<T, NZ, WC><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_zmid_reg<T, NZ, WC>, grid, nt, smem, s, a, a.pdl);
 }
 
 template <typename T, int NZ>
@@ -681,6 +684,7 @@ __device__ __forceinline__ void zpar_body(const YZArgs<T> &a, int bx, int ky)
 template <typename T, int NZ, int WC>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_zmid_par(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     zpar_body<T, NZ, WC>(a, blockIdx.x, blockIdx.y);
 }
@@ -697,8 +701,7 @@ static int launch_zmid_par_w(const YZArgs<T> &a, cudaStream_t s)
         if (e != cudaSuccess) return (int)e;
     }
     dim3 grid((a.LX + WC - 1) / WC, a.Ny / 2 + 1);
-    k_zmid_par<T, NZ, WC><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_zmid_par<T, NZ, WC>, grid, nt, smem, s, a, a.pdl);
 }
 
 template <typename T, int NZ>
@@ -807,6 +810,7 @@ __device__ __forceinline__ void ypass_prefetch_ahead(const YZArgs<T> &a, int L)
 template <typename T, int P, int Q, bool INV>
 __global__ void __launch_bounds__(yreg_maxt<T>::v) k_ypass_reg(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     if (a.pf_ahead > 0) ypass_prefetch_ahead<T, INV>(a, P * Q);
     ypass_reg_body<T, P, Q, INV>(a, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -856,8 +860,7 @@ static int launch_ypass_reg(const YZArgs<T> &a, cudaStream_t s)
     dim3 grid((a.LX + a.W - 1) / a.W, a.nz, 3);
     YZArgs<T> b = a;
     b.pf_ahead = resident_blocks(k_ypass_reg<T, P, Q, INV>, nt, smem);
-    k_ypass_reg<T, P, Q, INV><<<grid, nt, smem, s>>>(b);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_ypass_reg<T, P, Q, INV>, grid, nt, smem, s, b, b.pdl);
 }
 
 // ------------------------------------------------------------------------------ 2D y pass, two-level register FFT
@@ -1011,6 +1014,7 @@ __device__ __forceinline__ void ymid2d_reg_body(const YZArgs<T> &a, int bx)
 template <typename T, int P, int Q>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_ymid2d_reg(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     ymid2d_reg_body<T, P, Q>(a, blockIdx.x);
 }
@@ -1176,6 +1180,7 @@ __device__ __forceinline__ void ypass_st_body(const YZArgs<T> &a, int bx, int z,
 template <typename T, int L, bool INV>
 __global__ void __launch_bounds__(bm_lb<T>::v, sizeof(T) == 4 ? 2 : 1) k_ypass_st(YZArgs<T> a)
 {
+    pdl_enter();
     if (gated_out<T>(a.st, a.gate)) return;
     ypass_st_body<T, L, INV>(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
@@ -1209,8 +1214,7 @@ static int launch_ypass_st(const YZArgs<T> &a, cudaStream_t s)
         if (e != cudaSuccess) return (int)e;
     }
     dim3 grid((a.LX + a.W - 1) / a.W, a.nz, 3);
-    k_ypass_st<T, L, INV><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_ypass_st<T, L, INV>, grid, nt, smem, s, a, a.pdl);
 }
 
 template <typename T, bool INV>
@@ -1282,8 +1286,7 @@ static int launch_ymid2d_reg(const YZArgs<T> &a, cudaStream_t s)
     dim3 grid((a.LX + a.W - 1) / a.W);
     int rc = launch_common(k_ymid2d_reg<T, P, Q>, grid, nt, smem, s);
     if (rc) return rc;
-    k_ymid2d_reg<T, P, Q><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_ymid2d_reg<T, P, Q>, grid, nt, smem, s, a, a.pdl);
 }
 
 // the register 2D y pass for this tile width, or -1 when it does not apply
@@ -1325,8 +1328,7 @@ template <typename T> int launch_ymid2d(const YZArgs<T> &a, cudaStream_t s)
     dim3 grid((a.LX + a.W - 1) / a.W);
     int rc = launch_common(k_ymid2d<T>, grid, nt, smem, s);
     if (rc) return rc;
-    k_ymid2d<T><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_ymid2d<T>, grid, nt, smem, s, a, a.pdl);
 }
 
 template <typename T> int launch_yfwd(const YZArgs<T> &a, cudaStream_t s)
@@ -1350,8 +1352,7 @@ template <typename T> int launch_yfwd(const YZArgs<T> &a, cudaStream_t s)
     dim3 grid((a.LX + a.W - 1) / a.W, a.nz, 3);
     int rc = launch_common(k_ypass3d<T, false>, grid, nt, smem, s);
     if (rc) return rc;
-    k_ypass3d<T, false><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_ypass3d<T, false>, grid, nt, smem, s, a, a.pdl);
 }
 
 template <typename T> int launch_yinv(const YZArgs<T> &a, cudaStream_t s)
@@ -1375,8 +1376,7 @@ template <typename T> int launch_yinv(const YZArgs<T> &a, cudaStream_t s)
     dim3 grid((a.LX + a.W - 1) / a.W, a.nz, 3);
     int rc = launch_common(k_ypass3d<T, true>, grid, nt, smem, s);
     if (rc) return rc;
-    k_ypass3d<T, true><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_ypass3d<T, true>, grid, nt, smem, s, a, a.pdl);
 }
 
 template <typename T> int launch_zmid(const YZArgs<T> &a, cudaStream_t s)
@@ -1413,8 +1413,7 @@ template <typename T> int launch_zmid(const YZArgs<T> &a, cudaStream_t s)
     dim3 grid((a.LX + a.W - 1) / a.W, a.Ny / 2 + 1);
     int rc = launch_common(k_zmid<T>, grid, nt, smem, s);
     if (rc) return rc;
-    k_zmid<T><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_zmid<T>, grid, nt, smem, s, a, a.pdl);
 }
 
 

@@ -38,6 +38,7 @@ struct YZArgs {
     StepState *st;
     int gate;
     int yv;              // 3D y transform: 0 two-level register kernel, 1 radix-16 Stockham (Ny >= 256),
+    int pdl;             // launched with the programmatic dependence (launch_pdl)
                          // 2 the two-level kernel fed by bulk tensor copies (persistent, pipelined)
     int pf_ahead;        // set by the launchers: blocks of the grid resident at once (0: no look-ahead prefetch)
     int zv;              // 3D z pass: 0 one thread per pencil line, 1 the parity split (two threads per line)
@@ -148,6 +149,7 @@ struct StageArgs {
     int lte_embedded;    // LTE mode: the 5th-order solution recomputed in FP64 from the base and cev5 (nev 5)
     double cev5[6];      // LTE mode with lte_embedded: 5th-order weights of the same stage rhs as cev
     long long n;         // cells
+    int pdl;             // launched with the programmatic dependence (launch_pdl)
     int staged;          // prefetch the per-cell input rows into shared memory (register kernel)
     int xv;              // register x transform: 0 two-level P x Q, 1 radix-8 Stockham at 64 (FP32) registers
     // derived per-launch constants (products replace per-cell divisions)

@@ -711,6 +711,7 @@ template <typename T>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_stage(StageArgs<T> a)
 {
     if (stage_gated_out<T>(a.st, a.gate)) return;
+    pdl_enter();
     stage_generic_body<T>(a, blockIdx.x, gridDim.x);
 }
 
@@ -1112,6 +1113,7 @@ template <typename T, int LX, int SPEC>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx16(StageArgs<T> a)
 {
     if (stage_gated_out<T>(a.st, a.gate)) return;
+    pdl_enter();
     stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, gridDim.x);
 }
 
@@ -1119,6 +1121,7 @@ template <typename T, int LX, int SPEC>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX16_LO_MAXNREG_F) k_stage_rx16_lo(StageArgs<T> a)
 {
     if (stage_gated_out<T>(a.st, a.gate)) return;
+    pdl_enter();
     stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, gridDim.x);
 }
 
@@ -1126,6 +1129,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX16_LO_MAXNREG_F) k_stage
 // many meshes with the same x length in one launch (radix-8 transform): work item (mesh, row
 // block); the error-norm maximum and the step bookkeeping follow k_stage_batch
 template <typename T, int LX, int SPEC = 0>
+    pdl_enter();
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx_batch(const StageArgs<T> *__restrict__ args,
                                                                          const int2 *__restrict__ work, int nwork, unsigned int total)
 {
@@ -1133,6 +1137,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx_b
     const int2 it = work[blockIdx.x];
     stage_reg_body<T, LX, 1, SPEC>(args[it.x], it.y, total);
 }
+    pdl_enter();
 
 template <typename T, int LX, int XV>
 static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
@@ -1173,8 +1178,7 @@ static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
     }
     int nrows = a.ny * a.nz;
     dim3 grid((nrows + a.rpb - 1) / a.rpb);
-    kern<<<grid, nt, smem, s>>>(b);
-    return (int)cudaGetLastError();
+    return launch_pdl(kern, grid, nt, smem, s, b, b.pdl);
 }
 
 // the register stage kernels of one x-transform variant; -1: the variant has none of this length
@@ -1230,8 +1234,7 @@ template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s)
     }
     int nrows = a.ny * a.nz;
     dim3 grid((nrows + a.rpb - 1) / a.rpb);
-    k_stage<T><<<grid, nt, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return launch_pdl(k_stage<T>, grid, nt, smem, s, a, a.pdl);
 }
 
 
