@@ -78,7 +78,7 @@ struct Mesh {
     void *buf[4] = {nullptr, nullptr, nullptr, nullptr};   // A (M), P (sM1), B, C
     void *ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     void *S1 = nullptr, *S2 = nullptr, *K = nullptr;
-    void *twx = nullptr, *twx2 = nullptr, *twy = nullptr, *twz = nullptr;
+    void *twx = nullptr, *twx2 = nullptr, *twy = nullptr, *twz = nullptr, *twx4 = nullptr;
     void *Msd = nullptr, *K1d = nullptr, *Hout = nullptr;
     void *G = nullptr;          // evaluation speedup: es_level saved spectra (3 planes each)
     double es_cs[3] = {0, 0, 0};
@@ -206,7 +206,7 @@ void free_mesh(Mesh &m)
 {
     for (auto &p : m.buf) { if (p) cudaFree(p); p = nullptr; }
     for (auto &p : m.ev) { if (p) cudaFree(p); p = nullptr; }
-    void **ps[] = {&m.S1, &m.S2, &m.K, &m.twx, &m.twx2, &m.twy, &m.twz, &m.Msd, &m.K1d, &m.Hout, &m.G};
+    void **ps[] = {&m.S1, &m.S2, &m.K, &m.twx, &m.twx2, &m.twy, &m.twz, &m.twx4, &m.Msd, &m.K1d, &m.Hout, &m.G};
     for (auto pp : ps) { if (*pp) cudaFree(*pp); *pp = nullptr; }
     if (m.Had) cudaFree(m.Had);
     m.Had = nullptr;
@@ -303,6 +303,19 @@ int upload_table(void **dst, int L, bool fp64_only, cudaStream_t s)
         if (cudaMemcpyAsync(*dst, f.data(), bytes, cudaMemcpyHostToDevice, s) != cudaSuccess) return fail(BM_ECUDA, "twiddle upload");
         cudaStreamSynchronize(s);
     }
+    cudaStreamSynchronize(s);
+    return 0;
+}
+
+// tables of the FP32 x transforms on butterfly pairs (none for lengths without them)
+template <typename T> int upload_xpairs(void **dst, int LX, cudaStream_t s)
+{
+    if (sizeof(T) != 4) return 0;
+    const std::vector<float> tw = stage_pair_tables(LX);
+    if (tw.empty()) return 0;
+    if (cudaMalloc(dst, sizeof(float) * tw.size()) != cudaSuccess) return fail(BM_ENOMEM, "twiddle table allocation failed");
+    if (cudaMemcpyAsync(*dst, tw.data(), sizeof(float) * tw.size(), cudaMemcpyHostToDevice, s) != cudaSuccess)
+        return fail(BM_ECUDA, "twiddle upload");
     cudaStreamSynchronize(s);
     return 0;
 }
@@ -410,6 +423,7 @@ int prepare_mesh(bm_ctx *c, Mesh &m)
         if ((rc = upload_table<T>(&m.twx, m.LX, false, s))) return rc;
         if ((rc = upload_table<T>(&m.twx2, m.Nx, false, s))) return rc;
         if ((rc = upload_table<T>(&m.twy, m.Ny, false, s))) return rc;
+        if ((rc = upload_xpairs<T>(&m.twx4, m.LX, s))) return rc;
         if ((rc = upload_table<T>(&m.twz, m.Nz, false, s))) return rc;
     }
     if ((m.modules & BM_DEMAG) && m.ml_role == 0) {
@@ -531,6 +545,14 @@ float time_launches(cudaStream_t s, F launch, int reps)
 
 // Row counts per block the stage tuner tries: 1, and more while at least one block per SM remains (fewer
 // blocks only leave SMs idle: 7 blocks of 480 threads took 21 us where 64 blocks of one row took 10)
+template <typename T> bool tune_xv_ok(int LX, int xv)
+{
+    // x-transform variants a length has: 0 always (the generic kernel where there is no register one), 3 (radix
+    // 16 at the lower register cap) and 4 (butterfly pairs) in FP32
+    if (xv == 0) return true;
+    if (xv == 1) return stage_reg_q(LX, 1) != 0;
+    return stage_reg_q(LX, xv) != 0 && (xv == 2 || sizeof(T) == 4);
+}
 bool tune_rows_ok(int rows, int rpb) { return rpb == 1 || (rows + rpb - 1) / rpb >= 148; }
 
 // 3D y passes of one grid: transform variant (two-level register / radix-16 Stockham) x column
@@ -598,8 +620,9 @@ int tune_grid_x(bm_ctx *c, Mesh &G)
     h.Hout = tmp;
     float best = 1e30f; int br = G.rpb, bx = G.xv;
     const int rows = G.ny * G.nz;
-    for (int xv = 0; xv <= (stage_reg_q(G.LX, 2) ? (sizeof(T) == 4 ? 3 : 2) : 1); xv++)
+    for (int xv = 0; xv <= 4; xv++)
         for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
+            if (!tune_xv_ok<T>(G.LX, xv)) break;
             const int tpl = stage_reg_q(G.LX, xv) ? stage_reg_q(G.LX, xv) : G.px.tpl;
             if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
             if ((size_t)3 * rpb * padded_len(G.LX) * cs > 200 * 1024) break;
@@ -699,11 +722,12 @@ int autotune_mesh(bm_ctx *c, Mesh &m)
         const bool reg = stage_reg_q(m.LX, 1) != 0;
         // x-transform variant x rows per block x (per-cell rows prefetched to shared memory or
         // read from global); variants and staging apply to the register kernels only
-        for (int xv = 0; xv <= (stage_reg_q(m.LX, 2) ? (sizeof(T) == 4 ? 3 : 2) : reg ? 1 : 0); xv++)
-            for (int stg = 0; stg <= (reg ? 1 : 0); stg++)
+        for (int xv = 0; xv <= 4; xv++)
+            for (int stg = 0; stg <= (reg && xv < 4 ? 1 : 0); stg++)
                 for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
                     const int tpl = stage_reg_q(m.LX, xv) ? stage_reg_q(m.LX, xv) : m.px.tpl;
                     if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
+                    if (!tune_xv_ok<T>(m.LX, xv)) break;
                     if ((size_t)3 * rpb * padded_len(m.LX) * cs > 200 * 1024) break;
                     a.rpb = rpb;
                     a.staged = stg;
@@ -800,6 +824,7 @@ int prepare_grid(bm_ctx *c, Mesh &g)
     if ((rc = upload_table<T>(&g.twy, g.Ny, false, s))) return rc;
     if ((rc = upload_table<T>(&g.twz, g.Nz, false, s))) return rc;
     return 0;
+    if ((rc = upload_xpairs<T>(&g.twx4, g.LX, s))) return rc;
 }
 
 template <typename T>
@@ -1002,7 +1027,8 @@ int prepare_T(bm_ctx *c)
             m.staged = (sr && sr[0] == '1') ? 1 : 0;
             const char *sx = getenv("BM_STAGE_XV");
             m.xv = (sx && sx[0] == '1' && stage_reg_q(m.LX, 1)) ? 1 : (sx && sx[0] == '2' && stage_reg_q(m.LX, 2)) ? 2
-                 : (sx && sx[0] == '3' && stage_reg_q(m.LX, 2)) ? 3 : 0;
+                 : (sx && sx[0] == '3' && stage_reg_q(m.LX, 2)) ? 3
+                 : (sx && sx[0] == '4' && sizeof(T) == 4 && stage_reg_q(m.LX, 4)) ? 4 : 0;
             const char *sy = getenv("BM_Y_XV");
             m.yv = (sy && sy[0] == '1' && ypass_has_st(m.Ny) && m.nz > 1 && ypass_st_threads(m.Ny, m.Wy) % 32 == 0) ? 1 : 0;
             if (sy && sy[0] == '2' && m.nz > 1) {
@@ -1171,6 +1197,7 @@ int enqueue_yz(bm_ctx *c, Mesh &m, int gate, int *count)
         (*count)++;
     } else if (m.yzy) {
         CKL(launch_yzy<T>(a, c->stream), "yzy");
+    a.pdl = c->pdl;
         lt_mark(c, BM_TK_YZY, yz_alg_bytes(m, BM_TK_YZY, sizeof(T)));
         (*count)++;
     } else {
@@ -1197,7 +1224,6 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     a.S1 = (cpx<T> *)m.S1;
     a.twx = (const cpx<T> *)m.twx; a.twx2 = (const cpx<T> *)m.twx2;
     a.px = m.px;
-    a.pdl = c->pdl;
     a.rpb = m.rpb;
     a.scale = (T)(2.0 / ((double)m.Nx * m.Ny * m.Nz));
     a.modules = m.modules;
@@ -1212,6 +1238,7 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     a.do_xfwd = (m.modules & BM_DEMAG) ? 1 : 0;
     a.staged = m.staged;
     a.xv = m.xv;
+    a.twx4 = (const float4 *)m.twx4;
     for (int i = 0; i < 3; i++) a.pbc[i] = (m.pbc[i] > 0) - (m.pbc[i] < 0);
     stage_derive(a);
     if (m.ml_role == 2) {
@@ -1226,6 +1253,7 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
 
 template <typename T> T *B(Mesh &m, int i) { return (T *)m.buf[i]; }
 template <typename T> T *E(Mesh &m, int i) { return (T *)m.ev[i]; }
+    a.pdl = c->pdl;
 
 // Independent launches of a captured batched step as parallel branches of its graph: next() moves the
 // context to another side stream that waits for the fork point, join() brings the work back to the main
@@ -1253,7 +1281,6 @@ struct Branches {
             if (!(fork = event())) return fail(BM_ECUDA, "branch event");
             CK(cudaEventRecord(fork, main));
             return 0;
-    a.pdl = c->pdl;
         }
         const int k = turn++ % kSide;
         while ((int)c->side.size() <= k) {
@@ -2209,9 +2236,20 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
         if (rc) return rc;
     } else if (m.modules & BM_DEMAG) {
         StageArgs<T> a = stage_args<T>(c, m);
+// Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
+// latency between them (demag field of 32 x 16 x 1 cells 32 -> 28 us, of 200 x 150 x 12 in FP64 201 -> 191).
+// The captured steps don't take it: graph edges are as short already, and the next kernel's early blocks
+// cost the last wave of the one before (512 x 512 x 16 film, four RKDP54 steps 12.9 -> 13.4 ms).
+struct PdlScope {
+    bm_ctx *c;
+    explicit PdlScope(bm_ctx *ctx) : c(ctx) { c->pdl = true; }
+    ~PdlScope() { c->pdl = false; }
+};
+
         a.mode = BM_MODE_UPDATE;
         a.Min = B<T>(m, 0); a.Mbase = B<T>(m, 0);
         CKL(launch_stage<T>(a, c->stream), "xfwd");
+    PdlScope pdl(c);
         int rc = enqueue_yz<T>(c, m, BM_GATE_ALWAYS, &cnt);
         if (rc) return rc;
     }
@@ -2236,20 +2274,9 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
 // ------------------------------------------------------------------ discrete adjoint of RK4
 // Forward: the step graph with a checkpoint of M and the time every k steps. Backward, per segment
 // from the last: restore the checkpoint, replay a captured graph that recomputes the segment's k
-// Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
-// latency between them (demag field of 32 x 16 x 1 cells 32 -> 28 us, of 200 x 150 x 12 in FP64 201 -> 191).
-// The captured steps don't take it: graph edges are as short already, and the next kernel's early blocks
-// cost the last wave of the one before (512 x 512 x 16 film, four RKDP54 steps 12.9 -> 13.4 ms).
-struct PdlScope {
-    bm_ctx *c;
-    explicit PdlScope(bm_ctx *ctx) : c(ctx) { c->pdl = true; }
-    ~PdlScope() { c->pdl = false; }
-};
-
 // steps with the fused stage kernels also writing each stage's input, field and pre-normalisation
 // update into a k-slot cache, then replay a captured graph that walks the k steps in reverse
 // (renormalisation VJP, then per stage the LLG / local-field VJP, the demag of gH through the
-    PdlScope pdl(c);
 // convolution pipeline, and the Laplacian / accumulation kernel). Gradients accumulate in FP64;
 // the Zeeman gradient of each step is summed per step and mapped to its sample on the host with
 // the step start time the device used.
@@ -2894,6 +2921,7 @@ int demag_device_T(bm_ctx *c, Mesh &m, const S *M, S *H, int add, double *energy
     CKL(launch_stage<T>(h, s), "inverse x");
     double *dot = energy ? m.stage64 : nullptr;
     if (dot) CK(cudaMemsetAsync(dot, 0, sizeof(double), s));
+    PdlScope pdl(c);
     CKL((launch_planes_to_daos<S, T>(H, (const T *)m.Hout, m.n, add, M, dot, s)), "H out");
     if (dot) {
         double d = 0.0;
@@ -2921,7 +2949,6 @@ int get_m_device_T(bm_ctx *c, Mesh &m, void *M, int eb)
     else CKL((launch_planes_to_daos<double, T>((double *)M, B<T>(m, 0), m.n, 0, nullptr, nullptr, c->stream)), "M out");
     CK(cudaStreamSynchronize(c->stream));
     return 0;
-    PdlScope pdl(c);
 }
 
 int device_entry_checks(bm_ctx *c, int mesh, const void *p, int eb, void *stream)

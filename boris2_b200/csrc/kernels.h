@@ -1,5 +1,6 @@
 // Internal declarations shared by the kernel translation units and the host runtime.
 #pragma once
+#include <vector>
 #include "common.cuh"
 #include "fft.cuh"
 
@@ -37,8 +38,8 @@ struct YZArgs {
     int W;               // column tile width
     StepState *st;
     int gate;
-    int yv;              // 3D y transform: 0 two-level register kernel, 1 radix-16 Stockham (Ny >= 256),
     int pdl;             // launched with the programmatic dependence (launch_pdl)
+    int yv;              // 3D y transform: 0 two-level register kernel, 1 radix-16 Stockham (Ny >= 256),
                          // 2 the two-level kernel fed by bulk tensor copies (persistent, pipelined)
     int pf_ahead;        // set by the launchers: blocks of the grid resident at once (0: no look-ahead prefetch)
     int zv;              // 3D z pass: 0 one thread per pencil line, 1 the parity split (two threads per line)
@@ -127,6 +128,7 @@ struct StageArgs {
     const cpx<T> *twx2;  // length Nx (R2C split twiddles)
     FFTPlan px;
     int rpb;             // rows per block
+    const float4 *twx4;  // FP32, xv 4: the pair tables of xpair.cuh
     T scale;             // 2 / (Nx Ny Nz)
     int modules;
     T Ms, A, D, alpha, grel, K1, K2;
@@ -147,11 +149,12 @@ struct StageArgs {
     int renorm, mode, do_xfwd, last_kind, gate;
     int diag;            // BM_DIAG_* bits: this launch evaluates mxh / dmdt when requested, and publishes
     int lte_embedded;    // LTE mode: the 5th-order solution recomputed in FP64 from the base and cev5 (nev 5)
+    int pdl;             // launched with the programmatic dependence (launch_pdl)
     double cev5[6];      // LTE mode with lte_embedded: 5th-order weights of the same stage rhs as cev
     long long n;         // cells
-    int pdl;             // launched with the programmatic dependence (launch_pdl)
     int staged;          // prefetch the per-cell input rows into shared memory (register kernel)
-    int xv;              // register x transform: 0 two-level P x Q, 1 radix-8 Stockham at 64 (FP32) registers
+    int xv;              // register x transform: 0 two-level P x Q, 1 radix-8 Stockham at 64 (FP32) registers,
+                         // 2 radix 16, 3 radix 16 at the lower cap, 4 butterfly pairs (FP32)
     // derived per-launch constants (products replace per-cell divisions)
     T hh[3], ih[3], ih2[3];   // h, 1 / h, 1 / h^2
     T iMs;                    // 1 / Ms (uniform Ms)
@@ -228,6 +231,8 @@ int launch_yz_batch(int kind, int key, const YZArgs<T> *dargs, const int2 *dwork
                     cudaStream_t s);
 // key 0: generic-length stage kernel; key LX: the radix-8 register kernel of that length
 // the plain stage update of the RK stages (SPEC 1 of the radix-16 and batched register stage kernels):
+// the twiddle tables of xv 4 for x length LX (host; empty where it has none)
+std::vector<float> stage_pair_tables(int LX);
 // stage mode, exchange and demag on, the rhs and new M written, the new M's x transform; no saved
 // fields or states, no external field, no copy, no staging, no folded extrapolation
 template <typename T> inline bool stage_plain(const StageArgs<T> &a)

@@ -18,6 +18,7 @@
 #pragma once
 #include "kernels.h"
 #include "regfft.cuh"
+#include "xpair.cuh"
 
 template <typename T>
 __device__ __forceinline__ bool stage_gated_out(const StepState *st, int gate)
@@ -665,7 +666,7 @@ __device__ __forceinline__ void stage_tail(const StageArgs<T> &a, double lmax, u
 template <typename T>
 __device__ __forceinline__ void stage_generic_body(const StageArgs<T> &a, int bid, unsigned int total)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
     const int LX = a.LX, rpb = a.rpb, tpl = a.px.tpl;
     const int LSP = padded_len(LX);
@@ -710,8 +711,8 @@ __device__ __forceinline__ void stage_generic_body(const StageArgs<T> &a, int bi
 template <typename T>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_stage(StageArgs<T> a)
 {
-    if (stage_gated_out<T>(a.st, a.gate)) return;
     pdl_enter();
+    if (stage_gated_out<T>(a.st, a.gate)) return;
     stage_generic_body<T>(a, blockIdx.x, gridDim.x);
 }
 
@@ -774,6 +775,12 @@ template <int LX, int XV> struct xr_cfg {
     static constexpr int PAD = XV == 0 ? xr_pq<LX>::P : 16;   // one padding slot per PAD elements
     static constexpr int TPL = XV == 0 ? xr_pq<LX>::Q : xs_shape<LX, XV == 2 ? 16 : 8>::TPL;   // threads per line
     static constexpr int LSP = LX + LX / PAD + 1;             // padded line length
+};
+// xv 4: pairs of adjacent butterflies (xpair.cuh), elements in plain order
+template <int LX> struct xr_cfg<LX, 4> {
+    static constexpr int PAD = 1 << 20;
+    static constexpr int TPL = xp_shape<LX>::T;
+    static constexpr int LSP = xp_shape<LX>::LSP;
 };
 
 template <typename T, int P, int Q, bool INV>
@@ -968,7 +975,7 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
 {
     constexpr int SPEC = KS == 6 ? 1 : KS >= 4 ? 0 : KS;
     constexpr bool ODD = KS >= 5, STAGED = KS == 4;
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
     using C = xr_cfg<LX, XV>;
     constexpr int TPL = C::TPL, LSP = C::LSP;
@@ -983,8 +990,8 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
     cpx<T> *line = sm + (q < 3 * rpb ? q : 0) * LSP;
     const bool demag = SPEC == 1 || SPEC == 2 || (SPEC == 0 && (a.mode != BM_MODE_UPDATE) && (a.modules & BM_MOD_DEMAG));
     const int half = (a.nx + 1) >> 1;   // packed elements that carry mesh cells
-    // group 1: the spectrum rows
-    if (demag && qact) {
+    // group 1: the spectrum rows (xv 4 reads them straight into registers)
+    if (XV != 4 && demag && qact) {
         const cpx<T> *src = a.S1 + ((long long)qc * nrows + r0 + qr) * LX;
 #pragma unroll 4
         for (int m = t; m < LX; m += TPL) cp_async_cpx<T>(&line[A(m)], &src[m], true);
@@ -1045,9 +1052,11 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
     }
     cp_async_commit();
     if (demag) {
-        cp_async_wait_group<1>();
-        __syncthreads();
-        if (SPEC == 0 && a.es_fold) {
+        if constexpr (XV != 4) {
+            cp_async_wait_group<1>();
+            __syncthreads();
+        }
+        if (XV != 4 && SPEC == 0 && a.es_fold) {
             // evaluation speedup: an extrapolating evaluation turns the row of X[M] into the
             // extrapolated field's row (the k_es_extrap sum, formed here so the spectrum is not
             // written and read back); kept out of line so the hot path's registers are untouched
@@ -1056,9 +1065,13 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
                                             TPL);
             __syncthreads();
         }
-        if constexpr (XV == 0) xinv_pre_f<T>(line, LX, a.twx2, t, TPL, qact, A, [] { __syncthreads(); });
-        else xinv_pre_f<T>(line, LX, a.twx2, t, TPL, qact, A, [] { xs_sync<TPL>(); });
-        x_reg<T, LX, XV, true>(line, t, qact, a.twx, half);
+        if constexpr (XV == 4) {
+            xp_inverse<LX>(reinterpret_cast<float4 *>(line), a.S1 + ((long long)qc * nrows + r0 + qr) * LX, a.twx4, t, qact, half);
+        } else {
+            if constexpr (XV == 0) xinv_pre_f<T>(line, LX, a.twx2, t, TPL, qact, A, [] { __syncthreads(); });
+            else xinv_pre_f<T>(line, LX, a.twx2, t, TPL, qact, A, [] { xs_sync<TPL>(); });
+            x_reg<T, LX, XV, true>(line, t, qact, a.twx, half);
+        }
     }
     cp_async_wait_group<0>();
     __syncthreads();
@@ -1071,10 +1084,12 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
             if (mm >= half) sm[qq * LSP + A(mm)] = mk<T>(0, 0);
         }
         __syncthreads();
-        x_reg<T, LX, XV, false>(line, t, qact, a.twx, LX);
+        if constexpr (XV == 4)
+            xp_forward<LX>(reinterpret_cast<float4 *>(line), a.S1 + ((long long)qc * nrows + r0 + qr) * LX, a.twx4, t, qact);
+        else x_reg<T, LX, XV, false>(line, t, qact, a.twx, LX);
         // split into the packed half spectrum pairwise (k, LX - k) straight into the S1 row
         // (xfwd_post)
-        if (qact) {
+        if (XV != 4 && qact) {
             cpx<T> *dst = a.S1 + ((long long)qc * nrows + r0 + qr) * LX;
             for (int k = t; k <= LX / 2; k += TPL) {
                 if (k == 0) {
@@ -1098,6 +1113,7 @@ __device__ __forceinline__ void stage_reg_body(const StageArgs<T> &a, int bid, u
 template <typename T, int LX, int KS>
 __global__ void __launch_bounds__(bm_lb<T>::v) k_stage_reg(StageArgs<T> a)
 {
+    pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
     stage_reg_body<T, LX, 0, KS>(a, blockIdx.x, gridDim.x);
 }
@@ -1105,6 +1121,7 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_stage_reg(StageArgs<T> a)
 template <typename T, int LX, int KS>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx(StageArgs<T> a)
 {
+    pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
     stage_reg_body<T, LX, 1, KS>(a, blockIdx.x, gridDim.x);
 }
@@ -1112,24 +1129,36 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx(S
 template <typename T, int LX, int SPEC>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx16(StageArgs<T> a)
 {
-    if (stage_gated_out<T>(a.st, a.gate)) return;
     pdl_enter();
+    if (stage_gated_out<T>(a.st, a.gate)) return;
     stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, gridDim.x);
 }
 
 template <typename T, int LX, int SPEC>
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX16_LO_MAXNREG_F) k_stage_rx16_lo(StageArgs<T> a)
 {
-    if (stage_gated_out<T>(a.st, a.gate)) return;
     pdl_enter();
+    if (stage_gated_out<T>(a.st, a.gate)) return;
     stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, gridDim.x);
 }
 
 
+// register cap of the pair-transform kernels: stage launch of the 512 x 512 x 16 film 184 us at 72 (spills of
+// 16 to 64 bytes), 176 us at 80
+#ifndef BM_XP_MAXNREG
+#define BM_XP_MAXNREG 80
+#endif
+template <int LX, int KS>
+__global__ void __maxnreg__(BM_XP_MAXNREG) k_stage_xp(StageArgs<float> a)
+{
+    pdl_enter();
+    if (stage_gated_out<float>(a.st, a.gate)) return;
+    stage_reg_body<float, LX, 4, KS>(a, blockIdx.x, gridDim.x);
+}
+
 // many meshes with the same x length in one launch (radix-8 transform): work item (mesh, row
 // block); the error-norm maximum and the step bookkeeping follow k_stage_batch
 template <typename T, int LX, int SPEC = 0>
-    pdl_enter();
 __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx_batch(const StageArgs<T> *__restrict__ args,
                                                                          const int2 *__restrict__ work, int nwork, unsigned int total)
 {
@@ -1137,7 +1166,6 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx_b
     const int2 it = work[blockIdx.x];
     stage_reg_body<T, LX, 1, SPEC>(args[it.x], it.y, total);
 }
-    pdl_enter();
 
 template <typename T, int LX, int XV>
 static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
@@ -1168,6 +1196,9 @@ static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
         kern = b.staged ? k_stage_rx16<T, LX, 4> : odd ? (sp == 1 ? k_stage_rx16<T, LX, 6> : k_stage_rx16<T, LX, 5>)
              : sp == 1 ? k_stage_rx16<T, LX, 1> : sp == 2 ? k_stage_rx16<T, LX, 2> : sp == 3 ? k_stage_rx16<T, LX, 3>
                                                                                    : k_stage_rx16<T, LX, 0>;
+    else if constexpr (XV == 4)
+        kern = odd ? (sp == 1 ? k_stage_xp<LX, 6> : k_stage_xp<LX, 5>)
+             : sp == 1 ? k_stage_xp<LX, 1> : sp == 2 ? k_stage_xp<LX, 2> : sp == 3 ? k_stage_xp<LX, 3> : k_stage_xp<LX, 0>;
     else
         kern = b.staged ? k_stage_rx16_lo<T, LX, 4> : odd ? (sp == 1 ? k_stage_rx16_lo<T, LX, 6> : k_stage_rx16_lo<T, LX, 5>)
              : sp == 1 ? k_stage_rx16_lo<T, LX, 1> : sp == 2 ? k_stage_rx16_lo<T, LX, 2> : sp == 3 ? k_stage_rx16_lo<T, LX, 3>
@@ -1184,6 +1215,13 @@ static int launch_stage_reg(const StageArgs<T> &a, cudaStream_t s)
 // the register stage kernels of one x-transform variant; -1: the variant has none of this length
 template <typename T, int XV> int launch_stage_variant(const StageArgs<T> &a, cudaStream_t s)
 {
+    if constexpr (XV == 4) {
+        switch (a.LX) {
+        case 64: return launch_stage_reg<T, 64, XV>(a, s);
+        case 128: return launch_stage_reg<T, 128, XV>(a, s);
+        default: break;
+        }
+    }
     if constexpr (XV <= 1) {
         switch (a.LX) {
         case 16: return launch_stage_reg<T, 16, XV>(a, s);
@@ -1215,6 +1253,11 @@ template <typename T, int XV> int launch_stage_variant(const StageArgs<T> &a, cu
 template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s)
 {
     int rc = -1;
+    if constexpr (sizeof(T) == 4) {
+        // xv 4 has no staged rows and no folded extrapolation; those take the Stockham kernels
+        if (a.xv == 4 && !a.staged && !a.es_fold && a.twx4) rc = launch_stage_variant<T, 4>(a, s);
+        if (rc >= 0) return rc;
+    }
     if (a.LX >= 256 && a.LX % 3) {
         // xv 3 is its own kernel for FP32 only (the FP64 cap is the same for both)
         if constexpr (sizeof(T) == 4) {

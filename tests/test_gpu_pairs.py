@@ -1,11 +1,11 @@
 """Kernels that carry two x-adjacent values per thread, on cuda:0 against the oracle: the stage kernel's
 per-cell part on cell pairs (even and odd nx down to 1, every field term, open and periodic, each x
-transform variant).
+transform variant, the FP32 x transforms on butterfly pairs).
 Bounds as elsewhere: FP64 1e-9 and mixed 1e-5 of the largest field, states FP64 1e-9, mixed 1e-4 of Ms."""
 import numpy as np
 import pytest
 
-from oracle_libs import sphere_random, OracleSolver
+from oracle_libs import orc_hdemag, sphere_random, OracleSolver
 
 pytestmark = pytest.mark.gpu
 
@@ -20,8 +20,10 @@ def test_stage_pairs(bm, monkeypatch, nx, pbc, xv, prec, tol):
     d = dict(n=(nx, 5, 3), h=(4e-9, 3e-9, 2e-9), Ms=8e5, A=1.3e-11, D=1.5e-3, alpha=0.1, K1=1e5, K2=2e4, ea=(0.3, 0.2, 0.9),
              modules=1 | 4 | 8 | 16, Ha=(2e4, -1e4, 5e3), pbc=pbc)
     M = sphere_random(int(np.prod(d["n"])), seed=9 + nx, Ms=8e5)
+    # RKDP54 at a fixed step (dT_min = dT_max): adaptive steps scale with (error estimate)^(-1/6), so a
+    # mixed-precision estimate at its rounding floor would compare states at different times
     for ode in (0, 1):
-        s = OracleSolver([d], evaluation=ode, dt=2e-14)
+        s = OracleSolver([d], evaluation=ode, dt=2e-14, dT_min=2e-14, dT_max=2e-14)
         s.set_m(M)
         with bm.Context(precision=bm.FP64 if prec == "fp64" else bm.MIXED) as c:
             c.add_mesh(d["n"], d["h"])
@@ -30,10 +32,42 @@ def test_stage_pairs(bm, monkeypatch, nx, pbc, xv, prec, tol):
             c.set_pbc(0, pbc)
             c.set_field(0, d["Ha"])
             c.setode("RKDP54" if ode else "RK4", 2e-14)
+            if ode:
+                c.astepctrl(1e-4, 2.0, 2e-14, 2e-14)
             c.set_m(M)
             H, Href = c.update_field(), s.heff()
             assert np.abs(H - Href).max() / np.abs(Href).max() < (1e-9 if prec == "fp64" else 1e-5)
             c.run(6)
             s.run(6)
             assert np.abs(c.get_m() - s.get_m()).max() / 8e5 < tol
+        s.close()
+
+
+@pytest.mark.parametrize("nx", [49, 64, 100, 128, 201, 256, 401, 512, 1000])
+@pytest.mark.parametrize("rows", [1, 3])
+def test_stage_butterfly_pairs(bm, monkeypatch, nx, rows):
+    """The FP32 x transforms on butterfly pairs (BM_STAGE_XV=4): field, RK4 and RKDP54 steps."""
+    monkeypatch.setenv("BM_TILES", "1,1,4,%d" % (rows if nx < 600 else min(rows, 2)))
+    monkeypatch.setenv("BM_STAGE_XV", "4")
+    d = dict(n=(nx, 3, 2), h=(4e-9, 3e-9, 2e-9), Ms=8e5, A=1.3e-11, D=1.5e-3, alpha=0.1, K1=1e5, modules=1 | 4 | 8 | 16,
+             Ha=(2e4, -1e4, 5e3))
+    M = sphere_random(int(np.prod(d["n"])), seed=9 + nx, Ms=8e5)
+    for ode in (0, 1):
+        s = OracleSolver([d], evaluation=ode, dt=2e-14, dT_min=2e-14, dT_max=2e-14)
+        s.set_m(M)
+        with bm.Context(precision=bm.MIXED) as c:
+            c.add_mesh(d["n"], d["h"])
+            c.set_material(0, Ms=d["Ms"], A=d["A"], alpha=d["alpha"], K1=d["K1"], D=d["D"])
+            c.set_modules(0, d["modules"])
+            c.set_field(0, d["Ha"])
+            c.setode("RKDP54" if ode else "RK4", 2e-14)
+            if ode:
+                c.astepctrl(1e-4, 2.0, 2e-14, 2e-14)
+            c.set_m(M)
+            H, Href = c.demag_field(), orc_hdemag(M, d["n"], d["h"])[0]
+            assert c.tiles()["stage_xv"] == 4
+            assert np.abs(H - Href).max() / np.abs(Href).max() < 1e-5
+            c.run(6)
+            s.run(6)
+            assert np.abs(c.get_m() - s.get_m()).max() / 8e5 < 1e-4
         s.close()
