@@ -667,8 +667,10 @@ void tune_grid_yz(bm_ctx *c, Mesh &m)
                 if (zmid_has_reg(m.Nz) ? (zmid_reg_smem<T>(m.Nz, W) > 200 * 1024 || 6 * W > lim)
                                        : (zmid_smem<T>(m.Nz, W) > 200 * 1024 || 2 * W * m.pz.tpl > lim)) continue;
                 a.W = W;
-                // one thread per pencil line, and the parity split where it applies
-                for (int zv = 0; zv <= (zmid_has_par(m.Nz, W) ? 1 : 0); zv++) {
+                // one thread per pencil line, the parity split and the column pairs where they apply
+                for (int zv = 0; zv <= 2; zv++) {
+                    if (zv == 1 && !zmid_has_par(m.Nz, W)) continue;
+                    if (zv == 2 && !(sizeof(T) == 4 && zmid_has_pair(m.Nz, W, m.LX))) continue;
                     a.zv = zv;
                     float t = time_launches(s, [&]() { return launch_zmid<T>(a, s); }, reps);
                     if (t < best) { best = t; bw = W; bzv = zv; }
@@ -725,9 +727,9 @@ int autotune_mesh(bm_ctx *c, Mesh &m)
         for (int xv = 0; xv <= 4; xv++)
             for (int stg = 0; stg <= (reg && xv < 4 ? 1 : 0); stg++)
                 for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
+                    if (!tune_xv_ok<T>(m.LX, xv)) break;
                     const int tpl = stage_reg_q(m.LX, xv) ? stage_reg_q(m.LX, xv) : m.px.tpl;
                     if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
-                    if (!tune_xv_ok<T>(m.LX, xv)) break;
                     if ((size_t)3 * rpb * padded_len(m.LX) * cs > 200 * 1024) break;
                     a.rpb = rpb;
                     a.staged = stg;
@@ -822,9 +824,9 @@ int prepare_grid(bm_ctx *c, Mesh &g)
     if ((rc = upload_table<T>(&g.twx, g.LX, false, s))) return rc;
     if ((rc = upload_table<T>(&g.twx2, g.Nx, false, s))) return rc;
     if ((rc = upload_table<T>(&g.twy, g.Ny, false, s))) return rc;
+    if ((rc = upload_xpairs<T>(&g.twx4, g.LX, s))) return rc;
     if ((rc = upload_table<T>(&g.twz, g.Nz, false, s))) return rc;
     return 0;
-    if ((rc = upload_xpairs<T>(&g.twx4, g.LX, s))) return rc;
 }
 
 template <typename T>
@@ -1037,7 +1039,8 @@ int prepare_T(bm_ctx *c)
                 if (ypass_tma_fits<T>(ya)) m.yv = 2;
             }
             const char *szv = getenv("BM_Z_XV");
-            m.zv = (szv && szv[0] == '1' && m.nz > 1 && zmid_has_par(m.Nz, m.Wz)) ? 1 : 0;
+            m.zv = (szv && szv[0] == '1' && m.nz > 1 && zmid_has_par(m.Nz, m.Wz)) ? 1
+                 : (szv && szv[0] == '2' && m.nz > 1 && sizeof(T) == 4 && zmid_has_pair(m.Nz, m.Wz, m.LX)) ? 2 : 0;
             const char *sz = getenv("BM_YZY");
             m.yzy = 0;
             if (sz && sz[0] == '1' && m.nz > 1 && m.ml_role == 0 && (m.modules & BM_DEMAG) && !c->batched)
@@ -1194,10 +1197,10 @@ int enqueue_yz(bm_ctx *c, Mesh &m, int gate, int *count)
     if (m.nz == 1) {
         CKL(launch_ymid2d<T>(a, c->stream), "ymid2d");
         lt_mark(c, BM_TK_YMID2D, yz_alg_bytes(m, BM_TK_YMID2D, sizeof(T)));
+    a.pdl = c->pdl;
         (*count)++;
     } else if (m.yzy) {
         CKL(launch_yzy<T>(a, c->stream), "yzy");
-    a.pdl = c->pdl;
         lt_mark(c, BM_TK_YZY, yz_alg_bytes(m, BM_TK_YZY, sizeof(T)));
         (*count)++;
     } else {
@@ -1235,10 +1238,10 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     a.Ha = m.Had; a.nHa = m.nHa; a.Ha_tspan = m.Ha_tspan;
     a.st = c->st;
     a.n = m.n;
+    a.twx4 = (const float4 *)m.twx4;
     a.do_xfwd = (m.modules & BM_DEMAG) ? 1 : 0;
     a.staged = m.staged;
     a.xv = m.xv;
-    a.twx4 = (const float4 *)m.twx4;
     for (int i = 0; i < 3; i++) a.pbc[i] = (m.pbc[i] > 0) - (m.pbc[i] < 0);
     stage_derive(a);
     if (m.ml_role == 2) {
@@ -1250,10 +1253,10 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     }
     return a;
 }
+    a.pdl = c->pdl;
 
 template <typename T> T *B(Mesh &m, int i) { return (T *)m.buf[i]; }
 template <typename T> T *E(Mesh &m, int i) { return (T *)m.ev[i]; }
-    a.pdl = c->pdl;
 
 // Independent launches of a captured batched step as parallel branches of its graph: next() moves the
 // context to another side stream that waits for the fork point, join() brings the work back to the main
@@ -2233,9 +2236,6 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
             CKL(launch_stage<T>(a, c->stream), "xfwd");
         }
         int rc = enqueue_fields<T>(c, BM_GATE_ALWAYS, 0, &cnt);
-        if (rc) return rc;
-    } else if (m.modules & BM_DEMAG) {
-        StageArgs<T> a = stage_args<T>(c, m);
 // Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
 // latency between them (demag field of 32 x 16 x 1 cells 32 -> 28 us, of 200 x 150 x 12 in FP64 201 -> 191).
 // The captured steps don't take it: graph edges are as short already, and the next kernel's early blocks
@@ -2246,10 +2246,13 @@ struct PdlScope {
     ~PdlScope() { c->pdl = false; }
 };
 
+        if (rc) return rc;
+    } else if (m.modules & BM_DEMAG) {
+        StageArgs<T> a = stage_args<T>(c, m);
+    PdlScope pdl(c);
         a.mode = BM_MODE_UPDATE;
         a.Min = B<T>(m, 0); a.Mbase = B<T>(m, 0);
         CKL(launch_stage<T>(a, c->stream), "xfwd");
-    PdlScope pdl(c);
         int rc = enqueue_yz<T>(c, m, BM_GATE_ALWAYS, &cnt);
         if (rc) return rc;
     }
@@ -2918,10 +2921,10 @@ int demag_device_T(bm_ctx *c, Mesh &m, const S *M, S *H, int add, double *energy
     h.do_xfwd = 0;
     h.Min = B<T>(m, 0);
     h.Hout = (T *)m.Hout;
+    PdlScope pdl(c);
     CKL(launch_stage<T>(h, s), "inverse x");
     double *dot = energy ? m.stage64 : nullptr;
     if (dot) CK(cudaMemsetAsync(dot, 0, sizeof(double), s));
-    PdlScope pdl(c);
     CKL((launch_planes_to_daos<S, T>(H, (const T *)m.Hout, m.n, add, M, dot, s)), "H out");
     if (dot) {
         double d = 0.0;

@@ -14,6 +14,14 @@ bool zmid_has_par(int Nz, int W)
     return (Nz == 12 || Nz == 16 || Nz == 24 || Nz == 32 || Nz == 48 || Nz == 64) && (W == 8 || W == 16);
 }
 
+// whether the z pass on column pairs applies (FP32): even LX (16-byte rows), a register length up to 32, a
+// tile width of 8 to 64 within the shared memory
+bool zmid_has_pair(int Nz, int W, int LX)
+{
+    return LX % 2 == 0 && zmid_has_reg(Nz) && Nz <= 32 && (W == 8 || W == 16 || W == 32 || W == 64) &&
+           (size_t)6 * Nz * W * 8 + (size_t)6 * (Nz / 2 + 1) * (W + 1) * 4 + (size_t)6 * Nz * 8 + 16 <= 100 * 1024;
+}
+
 int ymid2d_reg_threads(int Ny, int W)
 {
     const int q = ysplit_q(Ny);

@@ -41,7 +41,7 @@ __device__ __forceinline__ void kapply(const T k[6], const cpx<T> m[3], cpx<T> h
 template <typename T>
 __device__ __forceinline__ void ymid2d_body(const YZArgs<T> &a, int bx)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     const int W = a.W, Ny = a.Ny, ny = a.ny, LX = a.LX;
     const int Ky1 = Ny / 2 + 1, Kx1 = LX + 1;
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_ymid2d_batch(const YZArgs<T> *_
 template <typename T, bool INV>
 __device__ __forceinline__ void ypass3d_body(const YZArgs<T> &a, int bx, int z, int c)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
     const int W = a.W, Ny = a.Ny, ny = a.ny, LX = a.LX, nz = a.nz;
     const int kx0 = bx * W;
@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_ypass3d_batch(const YZArgs<T> *
 template <typename T>
 __device__ __forceinline__ void zmid_body(const YZArgs<T> &a, int bx, int ky)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     const int W = a.W, Ny = a.Ny, Nz = a.Nz, nz = a.nz, LX = a.LX;
     const int Kx1 = LX + 1, Ky1 = Ny / 2 + 1, Kz1 = Nz / 2 + 1;
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_zmid_batch(const YZArgs<T> *__r
 template <typename T, int NZ, int WC>
 __device__ __forceinline__ void zmid_reg_body(const YZArgs<T> &a, int bx, int ky)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     const int W = WC ? WC : a.W, Ny = a.Ny, nz = a.nz, LX = a.LX;
     const int lw = WC ? (WC == 32 ? 5 : WC == 16 ? 4 : WC == 8 ? 3 : WC == 4 ? 2 : WC == 2 ? 1 : 0) : __ffs(W) - 1;
     constexpr int KZ1 = NZ / 2 + 1;
@@ -609,7 +609,7 @@ __device__ __forceinline__ void zpar_product(const YZArgs<T> &a, cpx<T> *v, cons
 template <typename T, int NZ, int WC>
 __device__ __forceinline__ void zpar_body(const YZArgs<T> &a, int bx, int ky)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int H = NZ / 2, KZ1 = NZ / 2 + 1;
     const int W = WC, Ny = a.Ny, nz = a.nz, LX = a.LX;
     constexpr int lw = WC == 16 ? 4 : 3;
@@ -723,7 +723,7 @@ static int launch_zmid_par(const YZArgs<T> &a, cudaStream_t s)
 template <typename T, int P, int Q, bool INV>
 __device__ __forceinline__ void ypass_reg_body(const YZArgs<T> &a, int bx, int z, int c)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     cpx<T> *sm = reinterpret_cast<cpx<T> *>(smraw);
     constexpr int L = P * Q;
     const int W = a.W, ny = a.ny, LX = a.LX, nz = a.nz;
@@ -891,7 +891,7 @@ __device__ __forceinline__ void y2d_stage1(const YZArgs<T> &a, cpx<T> *col, cpx<
 template <typename T, int P, int Q>
 __device__ __forceinline__ void ymid2d_reg_body(const YZArgs<T> &a, int bx)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     constexpr int Ny = P * Q, R = P > Q ? P : Q, Ky1 = Ny / 2 + 1;
     const int W = a.W, ny = a.ny, LX = a.LX;
     const int Kx1 = LX + 1;
@@ -1155,7 +1155,7 @@ __device__ __forceinline__ void ypass_st_pass(cpx<T> *tile, const cpx<T> *src, c
 template <typename T, int L, bool INV>
 __device__ __forceinline__ void ypass_st_body(const YZArgs<T> &a, int bx, int z, int c)
 {
-    extern __shared__ unsigned char smraw[];
+    extern __shared__ __align__(16) unsigned char smraw[];
     cpx<T> *tile = reinterpret_cast<cpx<T> *>(smraw);
     const int W = a.W, ny = a.ny, LX = a.LX, nz = a.nz;
     const int lw = __ffs(W) - 1;
@@ -1379,8 +1379,16 @@ template <typename T> int launch_yinv(const YZArgs<T> &a, cudaStream_t s)
     return launch_pdl(k_ypass3d<T, true>, grid, nt, smem, s, a, a.pdl);
 }
 
+#include "zpair.cuh"
+
 template <typename T> int launch_zmid(const YZArgs<T> &a, cudaStream_t s)
 {
+    if constexpr (sizeof(T) == 4) {
+        if (a.zv == 2) {
+            int rc = launch_zmid_pair(a, s);
+            if (rc >= 0) return rc;
+        }
+    }
     if (a.zv == 1 && zmid_has_par(a.Nz, a.W)) {
         switch (a.Nz) {
         case 12: return launch_zmid_par<T, 12>(a, s);

@@ -42,7 +42,8 @@ struct YZArgs {
     int yv;              // 3D y transform: 0 two-level register kernel, 1 radix-16 Stockham (Ny >= 256),
                          // 2 the two-level kernel fed by bulk tensor copies (persistent, pipelined)
     int pf_ahead;        // set by the launchers: blocks of the grid resident at once (0: no look-ahead prefetch)
-    int zv;              // 3D z pass: 0 one thread per pencil line, 1 the parity split (two threads per line)
+    int zv;              // 3D z pass: 0 one thread per pencil line, 1 the parity split (two threads per line),
+                         // 2 one thread per two adjacent pencil lines (FP32)
 };
 
 // Blocks of a launch resident on the whole GPU at once (occupancy per SM times the SMs), or 0 when
@@ -87,6 +88,7 @@ template <typename T> size_t zmid_reg_smem(int Nz, int W)
 }
 bool zmid_has_reg(int Nz);
 bool zmid_has_par(int Nz, int W);   // lengths and tile widths of the parity-split z pass
+bool zmid_has_pair(int Nz, int W, int LX);   // shapes of the FP32 z pass on column pairs
 bool ypass_has_reg(int Ny);
 // block-size ceiling of the two-level register y kernel: FP64 lines of 32 values need the registers
 // a 256-thread bound allows
@@ -126,9 +128,9 @@ struct StageArgs {
     cpx<T> *S1;
     const cpx<T> *twx;   // length LX
     const cpx<T> *twx2;  // length Nx (R2C split twiddles)
+    const float4 *twx4;  // FP32, xv 4: the pair tables of xpair.cuh
     FFTPlan px;
     int rpb;             // rows per block
-    const float4 *twx4;  // FP32, xv 4: the pair tables of xpair.cuh
     T scale;             // 2 / (Nx Ny Nz)
     int modules;
     T Ms, A, D, alpha, grel, K1, K2;
@@ -147,9 +149,9 @@ struct StageArgs {
     double cev[6];
     double crhs;
     int renorm, mode, do_xfwd, last_kind, gate;
+    int pdl;             // launched with the programmatic dependence (launch_pdl)
     int diag;            // BM_DIAG_* bits: this launch evaluates mxh / dmdt when requested, and publishes
     int lte_embedded;    // LTE mode: the 5th-order solution recomputed in FP64 from the base and cev5 (nev 5)
-    int pdl;             // launched with the programmatic dependence (launch_pdl)
     double cev5[6];      // LTE mode with lte_embedded: 5th-order weights of the same stage rhs as cev
     long long n;         // cells
     int staged;          // prefetch the per-cell input rows into shared memory (register kernel)
@@ -229,10 +231,10 @@ template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s);
 template <typename T>
 int launch_yz_batch(int kind, int key, const YZArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem,
                     cudaStream_t s);
-// key 0: generic-length stage kernel; key LX: the radix-8 register kernel of that length
-// the plain stage update of the RK stages (SPEC 1 of the radix-16 and batched register stage kernels):
 // the twiddle tables of xv 4 for x length LX (host; empty where it has none)
 std::vector<float> stage_pair_tables(int LX);
+// key 0: generic-length stage kernel; key LX: the radix-8 register kernel of that length
+// the plain stage update of the RK stages (SPEC 1 of the radix-16 and batched register stage kernels):
 // stage mode, exchange and demag on, the rhs and new M written, the new M's x transform; no saved
 // fields or states, no external field, no copy, no staging, no folded extrapolation
 template <typename T> inline bool stage_plain(const StageArgs<T> &a)

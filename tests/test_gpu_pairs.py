@@ -1,6 +1,7 @@
 """Kernels that carry two x-adjacent values per thread, on cuda:0 against the oracle: the stage kernel's
 per-cell part on cell pairs (even and odd nx down to 1, every field term, open and periodic, each x
-transform variant, the FP32 x transforms on butterfly pairs).
+transform variant, the FP32 x transforms on butterfly pairs) and the FP32 z pass on column pairs (BM_Z_XV=2;
+each length, partial tiles).
 Bounds as elsewhere: FP64 1e-9 and mixed 1e-5 of the largest field, states FP64 1e-9, mixed 1e-4 of Ms."""
 import numpy as np
 import pytest
@@ -71,3 +72,20 @@ def test_stage_butterfly_pairs(bm, monkeypatch, nx, rows):
             s.run(6)
             assert np.abs(c.get_m() - s.get_m()).max() / 8e5 < 1e-4
         s.close()
+
+
+@pytest.mark.parametrize("n,W", [((30, 7, 2), 8), ((16, 9, 3), 16), ((47, 6, 4), 32), ((100, 5, 6), 64), ((24, 12, 8), 16),
+                                 ((33, 8, 11), 8), ((64, 16, 13), 32), ((5, 4, 16), 8), ((128, 3, 9), 32)])
+def test_zpair_hdemag(bm, monkeypatch, n, W):
+    monkeypatch.setenv("BM_TILES", "1,1,%d,1" % W)
+    monkeypatch.setenv("BM_Z_XV", "2")
+    h = (3e-9, 2e-9, 2.5e-9)
+    M = sphere_random(int(np.prod(n)), seed=70 + n[0], Ms=8e5)
+    Href, _ = orc_hdemag(M, n, h)
+    with bm.Context(precision=bm.MIXED) as c:
+        c.add_mesh(n, h)
+        c.set_modules(0, bm.DEMAG)
+        c.set_m(M)
+        H = c.demag_field()
+        assert c.tiles()["zmid_zv"] == 2 and c.tiles()["zmid_W"] == W
+    assert np.abs(H - Href).max() / np.abs(Href).max() < 1e-5
