@@ -104,7 +104,7 @@ struct MLRun {
     std::vector<void *> in_w;
     void *K = nullptr;
     void *twz = nullptr;
-    int W = 8;
+    int W = 8, vec = 0;             // z pass: tile width, whole vectors per thread
     long long ncc = 0;
     // supermesh demag (BM_ML_SUPERMESH): one demag grid over the meshes' bounding box
     bool sm = false;
@@ -996,16 +996,29 @@ int prepare_ml(bm_ctx *c)
     const char *fw = getenv("BM_ML_W");   // fixed width (profiling runs)
     if (fw && atoi(fw) >= 1 && (atoi(fw) & (atoi(fw) - 1)) == 0) {
         r.W = atoi(fw);
+        const char *fv = getenv("BM_ML_VEC");   // with a fixed width: "1" the whole-vector form where it applies
+        r.vec = 0;
+        if (fv && fv[0] == '1') r.vec = zmid_ml_has_vec<T>(ml_zargs<T>(c, r.W, BM_GATE_ALWAYS)) ? 1 : 0;
         return 0;
     }
+    r.vec = 0;
     for (int W = 1; W <= 32 && W <= LX; W *= 2) {
         MLZArgs<T> z = ml_zargs<T>(c, W, BM_GATE_ALWAYS);
         z.st = nullptr;
         if (((6 * L * W + 31) & ~31) > lim || zmid_ml_smem<T>(L, g.N[2], W, z.ksm) > 200 * 1024) continue;
         if (!r.W) r.W = W;
         if (!c->autotune) continue;
+        z.vec = 0;
         float t = time_launches(s, [&]() { return launch_zmid_ml<T>(z, s); }, 3);
         if (t < best) { best = t; r.W = W; }
+    }
+    for (int W = 8; W <= 64 && W <= LX && c->autotune; W *= 2) {
+        MLZArgs<T> z = ml_zargs<T>(c, W, BM_GATE_ALWAYS);
+        z.st = nullptr;
+        z.vec = 1;
+        if (!zmid_ml_has_vec<T>(z)) continue;
+        float t = time_launches(s, [&]() { return launch_zmid_ml<T>(z, s); }, 3);
+        if (t < best) { best = t; r.W = W; r.vec = 1; }
     }
     if (!r.W) return fail(BM_EUNSUPPORTED, "multilayer: no z-pass tile fits");
     cudaGetLastError();
@@ -1184,6 +1197,7 @@ YZArgs<T> yz_args(bm_ctx *c, Mesh &m, int gate)
     a.nx = m.nx; a.ny = m.ny; a.nz = m.nz; a.LX = m.LX; a.Ny = m.Ny; a.Nz = m.Nz;
     a.W = m.nz > 1 ? m.Wy : m.W2;
     a.st = c->st; a.gate = gate;
+    a.pdl = c->pdl;
     a.yv = m.yv;
     a.zv = m.zv;
     return a;
@@ -1197,7 +1211,6 @@ int enqueue_yz(bm_ctx *c, Mesh &m, int gate, int *count)
     if (m.nz == 1) {
         CKL(launch_ymid2d<T>(a, c->stream), "ymid2d");
         lt_mark(c, BM_TK_YMID2D, yz_alg_bytes(m, BM_TK_YMID2D, sizeof(T)));
-    a.pdl = c->pdl;
         (*count)++;
     } else if (m.yzy) {
         CKL(launch_yzy<T>(a, c->stream), "yzy");
@@ -1225,6 +1238,7 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     a.nx = m.nx; a.ny = m.ny; a.nz = m.nz; a.LX = m.LX; a.Nx = m.Nx;
     a.hx = m.h[0]; a.hy = m.h[1]; a.hz = m.h[2];
     a.S1 = (cpx<T> *)m.S1;
+    a.twx4 = (const float4 *)m.twx4;
     a.twx = (const cpx<T> *)m.twx; a.twx2 = (const cpx<T> *)m.twx2;
     a.px = m.px;
     a.rpb = m.rpb;
@@ -1238,8 +1252,8 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     a.Ha = m.Had; a.nHa = m.nHa; a.Ha_tspan = m.Ha_tspan;
     a.st = c->st;
     a.n = m.n;
-    a.twx4 = (const float4 *)m.twx4;
     a.do_xfwd = (m.modules & BM_DEMAG) ? 1 : 0;
+    a.pdl = c->pdl;
     a.staged = m.staged;
     a.xv = m.xv;
     for (int i = 0; i < 3; i++) a.pbc[i] = (m.pbc[i] > 0) - (m.pbc[i] < 0);
@@ -1253,7 +1267,6 @@ StageArgs<T> stage_args(bm_ctx *c, Mesh &m)
     }
     return a;
 }
-    a.pdl = c->pdl;
 
 template <typename T> T *B(Mesh &m, int i) { return (T *)m.buf[i]; }
 template <typename T> T *E(Mesh &m, int i) { return (T *)m.ev[i]; }
@@ -1608,6 +1621,7 @@ MLZArgs<T> ml_zargs(bm_ctx *c, int W, int gate)
     z.twz = (const cpx<T> *)r.twz;
     z.L = L; z.nz = g.nc[2]; z.Ny = g.N[1]; z.Nz = g.N[2]; z.LX = g.N[0] / 2; z.W = W;
     z.st = c->st; z.gate = gate;
+    z.vec = r.vec;
     return z;
 }
 
@@ -2222,9 +2236,20 @@ int run_T(bm_ctx *c, int steps)
     return 0;
 }
 
+// Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
+// latency between them (demag field of 32 x 16 x 1 cells 32 -> 28 us, of 200 x 150 x 12 in FP64 201 -> 191).
+// The captured steps don't take it: graph edges are as short already, and the next kernel's early blocks
+// cost the last wave of the one before (512 x 512 x 16 film, four RKDP54 steps 12.9 -> 13.4 ms).
+struct PdlScope {
+    bm_ctx *c;
+    explicit PdlScope(bm_ctx *ctx) : c(ctx) { c->pdl = true; }
+    ~PdlScope() { c->pdl = false; }
+};
+
 template <typename T>
 int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
 {
+    PdlScope pdl(c);
     int cnt = 0;
     if ((m.modules & BM_DEMAG) && m.ml_role) {
         // x transforms of the layers that live on their mesh's grid, then the whole convolution
@@ -2236,20 +2261,9 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
             CKL(launch_stage<T>(a, c->stream), "xfwd");
         }
         int rc = enqueue_fields<T>(c, BM_GATE_ALWAYS, 0, &cnt);
-// Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
-// latency between them (demag field of 32 x 16 x 1 cells 32 -> 28 us, of 200 x 150 x 12 in FP64 201 -> 191).
-// The captured steps don't take it: graph edges are as short already, and the next kernel's early blocks
-// cost the last wave of the one before (512 x 512 x 16 film, four RKDP54 steps 12.9 -> 13.4 ms).
-struct PdlScope {
-    bm_ctx *c;
-    explicit PdlScope(bm_ctx *ctx) : c(ctx) { c->pdl = true; }
-    ~PdlScope() { c->pdl = false; }
-};
-
         if (rc) return rc;
     } else if (m.modules & BM_DEMAG) {
         StageArgs<T> a = stage_args<T>(c, m);
-    PdlScope pdl(c);
         a.mode = BM_MODE_UPDATE;
         a.Min = B<T>(m, 0); a.Mbase = B<T>(m, 0);
         CKL(launch_stage<T>(a, c->stream), "xfwd");
@@ -2907,6 +2921,7 @@ namespace {
 template <typename T, typename S>
 int demag_device_T(bm_ctx *c, Mesh &m, const S *M, S *H, int add, double *energy)
 {
+    PdlScope pdl(c);
     cudaStream_t s = c->stream;
     CKL((launch_daos_to_planes<S, T>(B<T>(m, 0), M, m.n, s)), "M in");
     StageArgs<T> a = stage_args<T>(c, m);
@@ -2921,7 +2936,6 @@ int demag_device_T(bm_ctx *c, Mesh &m, const S *M, S *H, int add, double *energy
     h.do_xfwd = 0;
     h.Min = B<T>(m, 0);
     h.Hout = (T *)m.Hout;
-    PdlScope pdl(c);
     CKL(launch_stage<T>(h, s), "inverse x");
     double *dot = energy ? m.stage64 : nullptr;
     if (dot) CK(cudaMemsetAsync(dot, 0, sizeof(double), s));

@@ -341,6 +341,234 @@ static int launch_zmid_ml_t(const MLZArgs<T> &a, cudaStream_t s)
     return a.W == 16 ? launch_zmid_ml_w<T, NZ, 16>(a, s) : launch_zmid_ml_w<T, NZ, 0>(a, s);
 }
 
+// ------------------------------------------------------------------------------ z pass, whole vectors per thread
+// For short z lines without full (in-plane shifted) kernels: thread (l, w), w fastest, owns all three
+// components of layer l on both mirror pencils of column w. The one-line form above reads two shared values
+// (an input and a kernel value) per complex product: shared-memory bandwidth bounds it (three layers, Nz = 4:
+// 9.5 GB of shared reads for 0.49 GB of spectra, 811 us at 1024 x 1024 x 2 cells). Here the six outputs a
+// thread accumulates share every input and every kernel value they use (K is symmetric, and the pencils
+// ky, -ky share |K|), a third of the shared reads, and the kernel values come straight from global memory:
+// a (destination, source) pair of layers uses its kernel once per column, so staging it would only copy it.
+// Measured (three layers, 1024 x 1024 x 2 cells, FFT 2048 x 2048 x 4): 811 -> 613 us, 2.59 TB/s of its 1.59 GB.
+// Signs: stored values hold ky, kz >= 0. kz > Nz / 2 takes the conjugate (xx, yy, zz, xy) or minus the
+// conjugate (xz, yz); ky < 0 changes the sign of xy and yz; a kernel computed for the opposite z shift that
+// of xz and yz (a self kernel is real).
+template <typename T, int NZ> struct MLVec {
+    static constexpr int KZ1 = NZ / 2 + 1;
+    // out[c][p][kz] += row products of one source layer; k6: the six components at akz, in: [c][p] at kz
+    template <int KZ, bool REAL>
+    __device__ __forceinline__ static void add(const cpx<T> k6[6], const cpx<T> in[3][2], cpx<T> out[3][2][NZ])
+    {
+        constexpr bool hi = KZ > NZ / 2;
+        constexpr int q[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int cc = 0; cc < 3; cc++) {
+                const int g = q[c][cc];
+                const bool oddz = g >= 4, oddy = g == 3 || g == 5;
+                // (re, im) of the value at this kz from the stored one
+                T kr = hi && oddz ? -k6[g].x : k6[g].x;
+                T ki = hi && !oddz ? -k6[g].y : k6[g].y;
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    const T r = (p && oddy) ? -kr : kr, i = (p && oddy) ? -ki : ki;
+                    const cpx<T> x = in[cc][p];
+                    cpx<T> &o = out[c][p][KZ];
+                    if (REAL) o = mk<T>(o.x + r * x.x, o.y + r * x.y);
+                    else o = mk<T>(o.x + r * x.x - i * x.y, o.y + r * x.y + i * x.x);
+                }
+            }
+    }
+};
+
+// the six stored components of unique kernel d at (akz, |ky|, kx)
+template <typename T>
+__device__ __forceinline__ void ml_k6(const MLZArgs<T> &a, const MLUDesc &d, bool inv, long long nk, long long at, cpx<T> k6[6])
+{
+    const T s = inv ? (T)-1 : (T)1;
+    if (d.kind == BM_MLK_SELF) {
+        const T *K = a.K + d.off + at;
+#pragma unroll
+        for (int g = 0; g < 6; g++) k6[g] = mk<T>(g >= 4 ? s * K[g * nk] : K[g * nk], (T)0);
+    } else {
+        const cpx<T> *K = reinterpret_cast<const cpx<T> *>(a.K + d.off) + at;
+#pragma unroll
+        for (int g = 0; g < 6; g++) {
+            k6[g] = K[g * nk];
+            if (g >= 4) k6[g] = cscale(k6[g], s);
+        }
+    }
+}
+
+template <typename T, int NZ, int KZ>
+__device__ __forceinline__ void ml_vec_kz(const cpx<T> k6[6], bool real, const cpx<T> *in, int W, cpx<T> out[3][2][NZ])
+{
+    cpx<T> x[3][2];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int p = 0; p < 2; p++) x[c][p] = in[((c * 2 + p) * NZ + KZ) * W];
+    if (real) MLVec<T, NZ>::template add<KZ, true>(k6, x, out);
+    else MLVec<T, NZ>::template add<KZ, false>(k6, x, out);
+}
+template <typename T, int NZ, int AKZ>
+__device__ __forceinline__ void ml_vec_src(const MLZArgs<T> &a, const MLUDesc &d, bool inv, long long nk, long long at, long long kzs,
+                                           const cpx<T> *in, int W, cpx<T> out[3][2][NZ])
+{
+    if constexpr (AKZ <= NZ / 2) {
+        cpx<T> k6[6];
+        ml_k6<T>(a, d, inv, nk, at + AKZ * kzs, k6);
+        const bool real = d.kind == BM_MLK_SELF;
+        ml_vec_kz<T, NZ, AKZ>(k6, real, in, W, out);
+        if constexpr (AKZ > 0 && 2 * AKZ < NZ) ml_vec_kz<T, NZ, NZ - AKZ>(k6, real, in, W, out);
+        ml_vec_src<T, NZ, AKZ + 1>(a, d, inv, nk, at, kzs, in, W, out);
+    }
+}
+
+template <typename T, int NZ>
+__global__ void __launch_bounds__(256) k_zmid_mlv(MLZArgs<T> a)
+{
+    if (ml_gated_out<T>(a.st, a.gate)) return;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    constexpr int KZ1 = NZ / 2 + 1, H = (NZ + 1) / 2;
+    const int W = a.W, L = a.L, Ny = a.Ny, nz = a.nz, LX = a.LX, lw = __ffs(W) - 1;
+    cpx<T> *In = reinterpret_cast<cpx<T> *>(smraw);                    // [L][3][2][NZ][W]
+    cpx<T> *O = In + (size_t)L * 6 * NZ * W;                           // column 0's outputs [L][3][2][NZ]
+    const int kx0 = blockIdx.x * W, ky = blockIdx.y, kym = ky == 0 ? 0 : Ny - ky;
+    const bool single = (ky == kym);
+    const int w = threadIdx.x & (W - 1), l = threadIdx.x >> lw, kx = kx0 + w;
+    const bool own = l < L && kx < LX;
+    const long long kzs = (long long)(Ny / 2 + 1) * (LX + 1), nk = kzs * KZ1, at = (long long)ky * (LX + 1) + kx;
+    const long long gstride = (long long)Ny * LX;
+    cpx<T> *S = a.S2[l < L ? l : 0];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            cpx<T> v[NZ];
+#pragma unroll
+            for (int e = 0; e < NZ; e++) v[e] = mk<T>(0, 0);
+            if (own && !(p && single)) {
+                const cpx<T> *src = S + ((long long)c * nz * Ny + (p ? kym : ky)) * LX + kx;
+#pragma unroll
+                for (int e = 0; e < H; e++)
+                    if (e < nz) v[e] = src[e * gstride];
+            }
+            RegFFT<T, NZ, false>::run(v, a.twz, 1);
+            if (l < L) {
+#pragma unroll
+                for (int e = 0; e < NZ; e++) In[(((l * 3 + c) * 2 + p) * NZ + e) * W + w] = v[e];
+            }
+        }
+    __syncthreads();
+    cpx<T> out[3][2][NZ];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int p = 0; p < 2; p++)
+#pragma unroll
+            for (int e = 0; e < NZ; e++) out[c][p][e] = mk<T>(0, 0);
+    if (own) {
+#pragma unroll 1
+        for (int s = 0; s < L; s++)
+            ml_vec_src<T, NZ, 0>(a, a.u[a.pu[l * L + s]], a.pinv[l * L + s] != 0, nk, at, kzs, In + (size_t)s * 6 * NZ * W + w, W,
+                                 out);
+    }
+    if (kx0 == 0) {
+        // column 0 packs the DC (kx = 0) and Nyquist (kx = Nx / 2) spectra: unpacked with the Hermitian mirror
+        // (pencil 0, kz) <-> (pencil pm, -kz), multiplied by their own kernel columns, re-packed
+        if (own && kx == 0) {
+            const int pm = single ? 0 : 1;
+#pragma unroll 1
+            for (int kz = 0; kz < NZ; kz++) {
+                const int kzm = (NZ - kz) % NZ, akz = kz <= NZ / 2 ? kz : NZ - kz;
+                const bool hi = kz > NZ / 2;
+                cpx<T> ap[3], bp[3];
+#pragma unroll
+                for (int c = 0; c < 3; c++) ap[c] = bp[c] = mk<T>(0, 0);
+#pragma unroll 1
+                for (int s = 0; s < L; s++) {
+                    const MLUDesc d = a.u[a.pu[l * L + s]];
+                    const bool inv = a.pinv[l * L + s] != 0;
+                    cpx<T> k0[6], kn[6];
+                    ml_k6<T>(a, d, inv, nk, at + akz * kzs, k0);
+                    ml_k6<T>(a, d, inv, nk, at + akz * kzs + LX, kn);
+#pragma unroll
+                    for (int g = 0; g < 6; g++)
+                        if (hi) {
+                            k0[g] = g >= 4 ? mk<T>(-k0[g].x, k0[g].y) : conj(k0[g]);
+                            kn[g] = g >= 4 ? mk<T>(-kn[g].x, kn[g].y) : conj(kn[g]);
+                        }
+                    constexpr int q[3][3] = {{0, 3, 4}, {3, 1, 5}, {4, 5, 2}};
+                    const cpx<T> *in = In + (size_t)s * 6 * NZ * W;
+#pragma unroll
+                    for (int cc = 0; cc < 3; cc++) {
+                        const cpx<T> C = in[((cc * 2) * NZ + kz) * W], cj = conj(in[((cc * 2 + pm) * NZ + kzm) * W]);
+                        const cpx<T> A = cscale(C + cj, (T)0.5), B = cscale(mul_mi(C - cj), (T)0.5);
+#pragma unroll
+                        for (int c = 0; c < 3; c++) {
+                            ap[c] = ap[c] + cmul(k0[q[c][cc]], A);
+                            bp[c] = bp[c] + cmul(kn[q[c][cc]], B);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    O[((l * 3 + c) * 2) * NZ + kz] = ap[c] + mul_i(bp[c]);
+                    if (!single) O[((l * 3 + c) * 2 + 1) * NZ + kzm] = conj(ap[c]) + mul_i(conj(bp[c]));
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++)
+#pragma unroll
+                for (int p = 0; p < 2; p++)
+#pragma unroll
+                    for (int e = 0; e < NZ; e++)
+                        if (!(p && single)) out[c][p][e] = O[((l * 3 + c) * 2 + p) * NZ + e];
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+        for (int p = 0; p < 2; p++) {
+            RegFFT<T, NZ, true>::run(out[c][p], a.twz, 1);
+            if (own && !(p && single)) {
+                cpx<T> *dst = S + ((long long)c * nz * Ny + (p ? kym : ky)) * LX + kx;
+#pragma unroll
+                for (int e = 0; e < H; e++)
+                    if (e < nz) dst[e * gstride] = out[c][p][e];
+            }
+        }
+}
+
+template <typename T> size_t zmid_mlv_smem(int L, int Nz, int W) { return (size_t)L * 6 * Nz * (W + 1) * sizeof(cpx<T>); }
+
+// whether the whole-vector form applies: z lines that fit the registers (FP32 up to 8 points, FP64 up to 4), no
+// full kernels, whole warps of at most 256 threads
+template <typename T> bool zmid_ml_has_vec(const MLZArgs<T> &a)
+{
+    if (!(a.Nz == 1 || a.Nz == 4 || (sizeof(T) == 4 && (a.Nz == 6 || a.Nz == 8)))) return false;
+    for (int u = 0; u < a.nu; u++)
+        if (a.u[u].kind == BM_MLK_FULL) return false;
+    return a.W >= 8 && (a.W & (a.W - 1)) == 0 && a.L * a.W <= 256 && zmid_mlv_smem<T>(a.L, a.Nz, a.W) <= 100 * 1024;
+}
+
+template <typename T, int NZ> static int launch_zmid_mlv(const MLZArgs<T> &a, cudaStream_t s)
+{
+    const int nt = (a.L * a.W + 31) & ~31;
+    const size_t smem = zmid_mlv_smem<T>(a.L, NZ, a.W);
+    if (smem > BM_SMEM_DEFAULT_SAFE) {
+        cudaError_t e = cudaFuncSetAttribute(k_zmid_mlv<T, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, BM_SMEM_CAP);
+        if (e != cudaSuccess) return (int)e;
+    }
+    dim3 grid((a.LX + a.W - 1) / a.W, a.Ny / 2 + 1);
+    k_zmid_mlv<T, NZ><<<grid, nt, smem, s>>>(a);
+    return (int)cudaGetLastError();
+}
+template bool zmid_ml_has_vec<float>(const MLZArgs<float> &);
+template bool zmid_ml_has_vec<double>(const MLZArgs<double> &);
+
 bool zmid_ml_supported(int Nz)
 {
     return Nz == 1 || Nz == 4 || Nz == 6 || Nz == 8 || Nz == 12 || Nz == 16 || Nz == 24 || Nz == 32 || Nz == 48 || Nz == 64;
@@ -349,6 +577,11 @@ bool zmid_ml_supported(int Nz)
 template <typename T> int launch_zmid_ml(const MLZArgs<T> &a, cudaStream_t s)
 {
     if (a.W < 1 || (a.W & (a.W - 1)) || a.L < 1 || a.L > BM_ML_MAXL) return 301;
+    if (a.vec && zmid_ml_has_vec<T>(a)) {
+        if (a.Nz == 1) return launch_zmid_mlv<T, 1>(a, s);
+        if (a.Nz == 4) return launch_zmid_mlv<T, 4>(a, s);
+        if constexpr (sizeof(T) == 4) return a.Nz == 6 ? launch_zmid_mlv<T, 6>(a, s) : launch_zmid_mlv<T, 8>(a, s);
+    }
     switch (a.Nz) {
     case 1: return launch_zmid_ml_t<T, 1>(a, s);
     case 4: return launch_zmid_ml_t<T, 4>(a, s);

@@ -117,6 +117,7 @@ struct MLZArgs {
     const cpx<T> *twz;
     int L, nu, nz, Ny, Nz, LX, W;
     int ksm;                  // bytes of staged kernel tiles
+    int vec;                  // whole vectors per thread (zmid_ml_has_vec) instead of one z line
     StepState *st;
     int gate;
 };
@@ -145,6 +146,7 @@ template <typename T> size_t zmid_ml_smem(int L, int Nz, int W, int ksm)
     return (size_t)L * 3 * 2 * Nz * W * sizeof(cpx<T>) + (size_t)ksm + (size_t)L * 6 * Nz * sizeof(cpx<T>);
 }
 template <typename T> int launch_zmid_ml(const MLZArgs<T> &a, cudaStream_t s);
+template <typename T> bool zmid_ml_has_vec(const MLZArgs<T> &a);   // shapes of the whole-vector z pass
 bool zmid_ml_supported(int Nz);
 
 // dst[c * dst_plane + i] = sum_q w[q] * src[idx[q] + c * src_plane], q in [ptr[i], ptr[i+1])
