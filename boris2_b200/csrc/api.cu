@@ -373,6 +373,30 @@ void choose_tiles(Mesh &m)
     }
 }
 
+// Meshes of a batch large enough to fill the GPU by themselves get launches of their own, as parallel branches
+// beside the work-list launches of the small ones: a work-list kernel reads its arguments from memory, takes
+// the block shape of the largest mesh of its group, and has no column-pair or butterfly-pair form.
+constexpr long long kSoloCells = 32768;
+bool batch_solo(const Mesh &m) { return m.n >= kSoloCells; }
+
+// tile shapes of a batch's large meshes without timing (a batch has hundreds of meshes to set up)
+template <typename T> void solo_tiles(Mesh &m)
+{
+    const bool f = sizeof(T) == 4;
+    m.xv = f && stage_reg_q(m.LX, 4) ? 4 : stage_reg_q(m.LX, 2) ? 2 : stage_reg_q(m.LX, 1) ? 1 : 0;
+    const int tpl = stage_reg_q(m.LX, m.xv) ? stage_reg_q(m.LX, m.xv) : m.px.tpl, rows = m.ny * m.nz;
+    m.rpb = std::max(1, std::min(96 / (3 * tpl), rows / 296));
+    if (m.nz == 1) {
+        m.W2 = 4;
+        while (m.W2 > 1 && (ymid2d_smem<T>(m.Ny, m.W2) > 110 * 1024 || m.W2 > m.LX || 3 * m.W2 * m.py.tpl > bm_lb<T>::v)) m.W2 /= 2;
+    } else if (f && m.Nz <= 16 && zmid_has_pair(m.Nz, 32, m.LX)) {
+        m.zv = 2;
+        m.Wz = 32;
+    } else {
+        while (m.Wz > 16) m.Wz /= 2;
+    }
+}
+
 template <typename T>
 int prepare_mesh(bm_ctx *c, Mesh &m)
 {
@@ -1058,7 +1082,11 @@ int prepare_T(bm_ctx *c)
             m.yzy = 0;
             if (sz && sz[0] == '1' && m.nz > 1 && m.ml_role == 0 && (m.modules & BM_DEMAG) && !c->batched)
                 m.yzy = yzy_available<T>(yz_args<T>(c, m, BM_GATE_ALWAYS)) == 0 ? 1 : 0;
-        } else if (c->autotune && !c->batched) autotune_mesh<T>(c, m);
+        } else if (c->batched) {
+            if (batch_solo(m)) solo_tiles<T>(m);
+        } else if (c->autotune) {
+            autotune_mesh<T>(c, m);
+        }
     }
     if (int rc = prepare_ml<T>(c)) { for (auto &mm : c->meshes) free_mesh(mm); free_ml(c); return rc; }
     return 0;
@@ -1413,16 +1441,31 @@ int stage_multi(bm_ctx *c, std::vector<StageArgs<T>> &v, int *count)
         a.diag |= pub;
     }
     std::map<int, std::vector<StageArgs<T>>> groups;   // x length with a register kernel, or 0
-    for (auto &a : v) groups[stage_reg_q(a.LX, 1) ? a.LX : 0].push_back(a);
-    const size_t first = c->bp.recs.size();
+    std::vector<StageArgs<T>> solo;
+    unsigned int total = 0;   // work items of the set: the large meshes' blocks and the work lists
+    for (auto &a : v) {
+        if (a.n < kSoloCells) {
+            groups[stage_reg_q(a.LX, 1) ? a.LX : 0].push_back(a);
+            continue;
+        }
+        solo.push_back(a);
+        total += (unsigned int)((a.ny * a.nz + a.rpb - 1) / a.rpb);
+    }
+    const size_t first = c->bp.collect ? c->bp.recs.size() : c->bp.next;
+    if (!c->bp.collect && !groups.empty() && first < c->bp.recs.size()) total = c->bp.recs[first].total;
     Branches br(c);
+    for (auto &a : solo) {
+        if (int rc = br.next()) return rc;
+        a.total = total;
+        if (!c->bp.collect) CKL(launch_stage<T>(a, c->stream), "stage");
+        (*count)++;
+    }
     for (auto &kv : groups) {
         if (int rc = br.next()) return rc;
         if (int rc = stage_batch_one<T>(c, kv.first, kv.second, count)) return rc;
     }
     if (int rc = br.join()) return rc;
     if (c->bp.collect) {
-        unsigned int total = 0;
         for (size_t i = first; i < c->bp.recs.size(); i++) total += (unsigned int)c->bp.recs[i].nwork;
         for (size_t i = first; i < c->bp.recs.size(); i++) c->bp.recs[i].total = total;
     }
@@ -1511,8 +1554,16 @@ int yz_multi(bm_ctx *c, int gate, int *count)
 {
     const int lim = 256;
     std::map<int, std::vector<YZArgs<T>>> g2, gy, gz;   // key Ny / Nz with a register kernel, or 0
+    Branches br(c);
+    int rc;
     for (auto &m : c->meshes) {
         if (!(m.modules & BM_DEMAG)) continue;
+        if (batch_solo(m)) {
+            if ((rc = br.next())) return rc;
+            if (c->bp.collect) continue;   // nothing to collect: launched with its own arguments
+            if ((rc = enqueue_yz<T>(c, m, gate, count))) return rc;
+            continue;
+        }
         YZArgs<T> a = yz_args<T>(c, m, gate);
         if (m.nz == 1) {
             // batched launches take their parallelism from the many meshes: wide column tiles
@@ -1556,12 +1607,10 @@ int yz_multi(bm_ctx *c, int gate, int *count)
             gz[0].push_back(a);
         }
     }
-    int rc;
     auto ykind = [](int key, bool inv) {
         return key > 0 ? (inv ? BM_BATCH_YINV_REG : BM_BATCH_YFWD_REG) : key < 0 ? (inv ? BM_BATCH_YINV_ST : BM_BATCH_YFWD_ST)
                                                                             : (inv ? BM_BATCH_YINV : BM_BATCH_YFWD);
     };
-    Branches br(c);
     for (auto &kv : gy) {
         if ((rc = br.next())) return rc;
         if ((rc = yz_batch_one<T>(c, ykind(kv.first, false), kv.first < 0 ? -kv.first : kv.first, kv.second, count))) return rc;

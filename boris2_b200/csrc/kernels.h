@@ -150,6 +150,7 @@ struct StageArgs {
     double crhs;
     int renorm, mode, do_xfwd, last_kind, gate;
     int pdl;             // launched with the programmatic dependence (launch_pdl)
+    unsigned int total;  // work items of the set of launches that finishes the step together (0: this launch's)
     int diag;            // BM_DIAG_* bits: this launch evaluates mxh / dmdt when requested, and publishes
     int lte_embedded;    // LTE mode: the 5th-order solution recomputed in FP64 from the base and cev5 (nev 5)
     double cev5[6];      // LTE mode with lte_embedded: 5th-order weights of the same stage rhs as cev

@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_stage(StageArgs<T> a)
 {
     pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_generic_body<T>(a, blockIdx.x, gridDim.x);
+    stage_generic_body<T>(a, blockIdx.x, a.total ? a.total : gridDim.x);
 }
 
 // many meshes in one launch: work item (mesh, row block). The meshes share the step state; every
@@ -1115,7 +1115,7 @@ __global__ void __launch_bounds__(bm_lb<T>::v) k_stage_reg(StageArgs<T> a)
 {
     pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_reg_body<T, LX, 0, KS>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<T, LX, 0, KS>(a, blockIdx.x, a.total ? a.total : gridDim.x);
 }
 
 template <typename T, int LX, int KS>
@@ -1123,7 +1123,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx(S
 {
     pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_reg_body<T, LX, 1, KS>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<T, LX, 1, KS>(a, blockIdx.x, a.total ? a.total : gridDim.x);
 }
 
 template <typename T, int LX, int SPEC>
@@ -1131,7 +1131,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX_MAXNREG_F) k_stage_rx16
 {
     pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, a.total ? a.total : gridDim.x);
 }
 
 template <typename T, int LX, int SPEC>
@@ -1139,7 +1139,7 @@ __global__ void __maxnreg__(sizeof(T) == 8 ? 128 : BM_RX16_LO_MAXNREG_F) k_stage
 {
     pdl_enter();
     if (stage_gated_out<T>(a.st, a.gate)) return;
-    stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<T, LX, 2, SPEC>(a, blockIdx.x, a.total ? a.total : gridDim.x);
 }
 
 
@@ -1153,7 +1153,7 @@ __global__ void __maxnreg__(BM_XP_MAXNREG) k_stage_xp(StageArgs<float> a)
 {
     pdl_enter();
     if (stage_gated_out<float>(a.st, a.gate)) return;
-    stage_reg_body<float, LX, 4, KS>(a, blockIdx.x, gridDim.x);
+    stage_reg_body<float, LX, 4, KS>(a, blockIdx.x, a.total ? a.total : gridDim.x);
 }
 
 // many meshes with the same x length in one launch (radix-8 transform): work item (mesh, row
