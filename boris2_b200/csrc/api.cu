@@ -575,6 +575,7 @@ template <typename T> bool tune_xv_ok(int LX, int xv)
     // 16 at the lower register cap) and 4 (butterfly pairs) in FP32
     if (xv == 0) return true;
     if (xv == 1) return stage_reg_q(LX, 1) != 0;
+    if (xv == 3 && stage_reg_q(LX, 4)) return false;   // the pairs are faster wherever the lower cap was
     return stage_reg_q(LX, xv) != 0 && (xv == 2 || sizeof(T) == 4);
 }
 bool tune_rows_ok(int rows, int rpb) { return rpb == 1 || (rows + rpb - 1) / rpb >= 148; }
@@ -743,26 +744,24 @@ int autotune_mesh(bm_ctx *c, Mesh &m)
         a.ev[0] = (const T *)m.buf[0]; a.ev[1] = (const T *)m.buf[0];
         a.ev_out = tmp;
         a.Mout = tmp + 3 * m.n;
-        float best = 1e30f; int br = m.rpb, bs = 0, bx = 0;
+        float best = 1e30f; int br = m.rpb, bx = 0;
         int rows = m.ny * m.nz;
-        const bool reg = stage_reg_q(m.LX, 1) != 0;
-        // x-transform variant x rows per block x (per-cell rows prefetched to shared memory or
-        // read from global); variants and staging apply to the register kernels only
+        // x-transform variant x rows per block (rows staged in shared memory are not tried: with cells in
+        // pairs they are slower at every size, 256 x 256 x 4 cells 46 against 27 us)
+        a.staged = 0;
         for (int xv = 0; xv <= 4; xv++)
-            for (int stg = 0; stg <= (reg && xv < 4 ? 1 : 0); stg++)
-                for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
-                    if (!tune_xv_ok<T>(m.LX, xv)) break;
-                    const int tpl = stage_reg_q(m.LX, xv) ? stage_reg_q(m.LX, xv) : m.px.tpl;
-                    if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
-                    if ((size_t)3 * rpb * padded_len(m.LX) * cs > 200 * 1024) break;
-                    a.rpb = rpb;
-                    a.staged = stg;
-                    a.xv = xv;
-                    float t = time_launches(s, [&]() { return launch_stage<T>(a, s); }, reps);
-                    if (t < best) { best = t; br = rpb; bs = stg; bx = xv; }
-                }
+            for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
+                if (!tune_xv_ok<T>(m.LX, xv)) break;
+                const int tpl = stage_reg_q(m.LX, xv) ? stage_reg_q(m.LX, xv) : m.px.tpl;
+                if (((3 * rpb * tpl + 31) & ~31) > lim || !tune_rows_ok(rows, rpb)) break;
+                if ((size_t)3 * rpb * padded_len(m.LX) * cs > 200 * 1024) break;
+                a.rpb = rpb;
+                a.xv = xv;
+                float t = time_launches(s, [&]() { return launch_stage<T>(a, s); }, reps);
+                if (t < best) { best = t; br = rpb; bx = xv; }
+            }
         m.rpb = br;
-        m.staged = bs;
+        m.staged = 0;
         m.xv = bx;
     }
     cudaStreamSynchronize(s);

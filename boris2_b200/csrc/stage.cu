@@ -55,11 +55,18 @@ std::vector<float> stage_pair_tables(int LX)
         t.push_back((float)(f * (double)sinl(two_pi * m0 / N)));
         t.push_back((float)(f * (double)sinl(two_pi * m1 / N)));
     };
-    for (int k = 0; k < LX; k += 2) put(k, k + 1, 2.0L * LX, 0.5);
-    for (int p = 1; p < xp_passes(LX); p++) {
+    // the split at the mirror butterflies (q, LR - q; 0 and LR / 2) of the first and of the last pass
+    const int last = xp_passes(LX) - 1, R0 = xp_radix(LX, 0), RL = xp_radix(LX, last);
+    for (int R : {R0, RL})
+        for (int r = 0, LR = LX / R; r < R; r++)
+            for (int q = 0; q < LR / 2; q++) put(q + r * LR, (q ? LR - q : LR / 2) + r * LR, 2.0L * LX, 0.5);
+    for (int p = 1; p <= last; p++) {
         const int R = xp_radix(LX, p), NS = xp_ns(LX, p);
         for (int r = 1; r < R; r++)
             for (int k = 0; k < NS; k += 2) put((long double)r * k, (long double)r * (k + 1), (long double)NS * R, 1.0);
     }
+    const int LR = LX / RL;
+    for (int r = 1; r < RL; r++)
+        for (int q = 0; q < LR / 2; q++) put((long double)r * q, (long double)r * (q ? LR - q : LR / 2), (long double)LX, 1.0);
     return t;
 }
