@@ -37,29 +37,47 @@ __device__ __forceinline__ void block_sum_add(double v, double *out)
     __syncthreads();
 }
 
+// (x, y, z) of cell i, in 32-bit arithmetic while the cell count allows it: the 64-bit divisions, with six
+// divisions by h^2 per component, were most of the cell kernels' 10 us on a 256 x 256 film
+template <typename T> __device__ __forceinline__ void adj_xyz(const AdjArgs<T> &a, long long i, int &x, int &y, int &z)
+{
+    if (a.n <= 0x7fffffffll) {
+        const unsigned u = (unsigned)i, q = u / (unsigned)a.nx, w = q / (unsigned)a.ny;
+        x = (int)(u - q * (unsigned)a.nx);
+        y = (int)(q - w * (unsigned)a.ny);
+        z = (int)w;
+    } else {
+        const long long q = i / a.nx, w = q / a.ny;
+        x = (int)(i - q * a.nx);
+        y = (int)(q - w * a.ny);
+        z = (int)w;
+    }
+}
+
+// neighbour of a cell along one axis minus its own value v: the cell at off, or at the missing side the far
+// cell (at far) times the axis' sign where periodic, else nothing
+template <typename T>
+__device__ __forceinline__ T adj_diff(const T *V, T v, bool in, long long off, int pbc, long long far)
+{
+    if (in) return V[off] - v;
+    return pbc ? (T)pbc * V[far] - v : (T)0;
+}
+
 // Neumann Laplacian of one component at cell (x, y, z): only existing neighbours; along a periodic
 // axis the far-side cell, times the axis' sign, stands in for the missing one (the operator stays
 // symmetric for either sign)
 template <typename T>
 __device__ __forceinline__ T adj_lap(const T *V, int x, int y, int z, long long cell, const AdjArgs<T> &a)
 {
-    const T v = V[cell];
-    T s = 0;
+    const T *C = V + cell;
+    const T v = *C;
     const long long nxy = (long long)a.nx * a.ny;
     const long long wx = a.nx - 1, wy = (long long)(a.ny - 1) * a.nx, wz = (long long)(a.nz - 1) * nxy;
-    const bool px = a.pbc[0] && a.nx > 1, py = a.pbc[1] && a.ny > 1, pz = a.pbc[2] && a.nz > 1;
-    if (x > 0) s += (V[cell - 1] - v) / (a.hx * a.hx);
-    else if (px) s += ((T)a.pbc[0] * V[cell + wx] - v) / (a.hx * a.hx);
-    if (x + 1 < a.nx) s += (V[cell + 1] - v) / (a.hx * a.hx);
-    else if (px) s += ((T)a.pbc[0] * V[cell - wx] - v) / (a.hx * a.hx);
-    if (y > 0) s += (V[cell - a.nx] - v) / (a.hy * a.hy);
-    else if (py) s += ((T)a.pbc[1] * V[cell + wy] - v) / (a.hy * a.hy);
-    if (y + 1 < a.ny) s += (V[cell + a.nx] - v) / (a.hy * a.hy);
-    else if (py) s += ((T)a.pbc[1] * V[cell - wy] - v) / (a.hy * a.hy);
-    if (z > 0) s += (V[cell - nxy] - v) / (a.hz * a.hz);
-    else if (pz) s += ((T)a.pbc[2] * V[cell + wz] - v) / (a.hz * a.hz);
-    if (z + 1 < a.nz) s += (V[cell + nxy] - v) / (a.hz * a.hz);
-    else if (pz) s += ((T)a.pbc[2] * V[cell - wz] - v) / (a.hz * a.hz);
+    const int px = a.nx > 1 ? a.pbc[0] : 0, py = a.ny > 1 ? a.pbc[1] : 0, pz = a.nz > 1 ? a.pbc[2] : 0;
+    const T dx = adj_diff(C, v, x > 0, -1, px, wx) + adj_diff(C, v, x + 1 < a.nx, 1, px, -wx);
+    const T dy = adj_diff(C, v, y > 0, -(long long)a.nx, py, wy) + adj_diff(C, v, y + 1 < a.ny, a.nx, py, -wy);
+    T s = dx * a.ih2[0] + dy * a.ih2[1];
+    if (a.nz > 1) s += (adj_diff(C, v, z > 0, -nxy, pz, wz) + adj_diff(C, v, z + 1 < a.nz, nxy, pz, -wz)) * a.ih2[2];
     return s;
 }
 
@@ -133,7 +151,8 @@ __global__ void k_adj_vjp_a(AdjArgs<T> a, const T *__restrict__ X, const T *__re
         double gms = -(double)pre * (double)a.alpha / ((double)Ms * Ms) * ((double)mx * xh - (double)mh * xx);
         if (a.modules & BM_MOD_EXCH) {
             const T cst = 2 * a.A / ((T)BM_MU0 * Ms * Ms);
-            const int xi = (int)(i % a.nx), yi = (int)((i / a.nx) % a.ny), zi = (int)(i / ((long long)a.nx * a.ny));
+            int xi, yi, zi;
+            adj_xyz(a, i, xi, yi, zi);
             double dot = 0.0;
             for (int c = 0; c < 3; c++) {
                 dot += (double)gh[c] * (double)adj_lap(X + c * n, xi, yi, zi, i, a);
@@ -171,7 +190,8 @@ __global__ void k_adj_vjp_c(AdjArgs<T> a, const T *__restrict__ gXd, const T *__
     const long long n = a.n;
     const bool exch = (a.modules & BM_MOD_EXCH) != 0;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int xi = (int)(i % a.nx), yi = (int)((i / a.nx) % a.ny), zi = (int)(i / ((long long)a.nx * a.ny));
+        int xi, yi, zi;
+        adj_xyz(a, i, xi, yi, zi);
         for (int c = 0; c < 3; c++) {
             T g = gXd[c * n + i];
             if (exch) g += adj_lap(w + c * n, xi, yi, zi, i, a);

@@ -2411,7 +2411,7 @@ int adjoint_T(bm_ctx *c, int steps, int k, const double *target, int m0_scales, 
     AdjArgs<T> aa;
     memset(&aa, 0, sizeof(aa));
     aa.nx = m.nx; aa.ny = m.ny; aa.nz = m.nz; aa.n = n;
-    aa.hx = (T)m.h[0]; aa.hy = (T)m.h[1]; aa.hz = (T)m.h[2];
+    for (int q = 0; q < 3; q++) aa.ih2[q] = (T)(1.0 / (m.h[q] * m.h[q]));
     aa.Ms_map = (const T *)m.Msd; aa.K1_map = (const T *)m.K1d;
     aa.Ms = (T)m.Ms; aa.K1 = (T)m.K1; aa.A = (T)m.A; aa.alpha = (T)m.alpha; aa.grel = (T)m.grel;
     double en = std::sqrt(m.ea[0] * m.ea[0] + m.ea[1] * m.ea[1] + m.ea[2] * m.ea[2]);

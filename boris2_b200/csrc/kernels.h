@@ -270,7 +270,7 @@ template <typename T>
 struct AdjArgs {
     int nx, ny, nz;
     long long n;
-    T hx, hy, hz;
+    T ih2[3];     // 1 / h^2 per axis
     const T *Ms_map, *K1_map;
     T Ms, K1, A, alpha, grel;
     T ea[3];
