@@ -174,6 +174,7 @@ struct bm_ctx {
     int kernels_per_step = 0;
     double *farq = nullptr;
     StepState host_st;
+    bool st_known = false;     // host_st equals the device's step state (nothing that writes it has run since)
     bool batched = false;       // many meshes per launch (work lists) instead of one launch per mesh
     BatchPlan bp;
     int ml_mode = -1;           // -1 off; 0 3D, 1 2D, 2 2D layered, 3 supermesh
@@ -515,16 +516,21 @@ int upload_state(bm_ctx *c)
     h.blocks_done = 0;
     h.mxh_acc = 0;
     h.dmdt_acc = 0;
+    // from pageable memory: host_st may change again once this returns
     CK(cudaMemcpyAsync(c->st, &h, sizeof(StepState), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
+    c->st_known = true;
     c->state_dirty = false;
     return 0;
 }
 
+// the device's step state in host_st. Only the steps and the calls that request a diagnostic change it, so between
+// them (bm_set_m, bm_set_ode, the statistics after a run) the copy at hand is current and no wait is needed
 int read_state(bm_ctx *c)
 {
+    if (c->st_known) return 0;
     CK(cudaMemcpyAsync(&c->host_st, c->st, sizeof(StepState), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
+    c->st_known = true;
     return 0;
 }
 
@@ -2268,6 +2274,7 @@ int run_T(bm_ctx *c, int steps)
             long long need = (long long)c->host_st.es_K - 1 - c->host_st.es_saved;
             warm = need > 0 ? (need < k ? need : k) : 0;
         }
+        c->st_known = false;
         for (long long i = 0; i < warm; i++) CK(cudaGraphLaunch(c->gexec, c->stream));
         for (long long i = warm; i < k; i++) CK(cudaGraphLaunch(c->gexec_es, c->stream));
         guard += k;
@@ -2380,6 +2387,7 @@ int adjoint_T(bm_ctx *c, int steps, int k, const double *target, int m0_scales, 
     }
     if (int rc = read_state(c)) return rc;
     const StepState st0 = c->host_st;
+    c->st_known = false;
     void *ckM = ab.get(v3 * S, false, s), *ckT = ab.get(sizeof(double) * S, false, s);
     if (!need(ckM) || !need(ckT)) return fail(BM_ENOMEM, "adjoint checkpoints");
     cudaEvent_t e0, e1, e2, e3;
@@ -2393,6 +2401,7 @@ int adjoint_T(bm_ctx *c, int steps, int k, const double *target, int m0_scales, 
     CK(cudaEventRecord(e1, s));
     if (int rc = read_state(c)) return rc;
     const StepState st_end = c->host_st;
+    c->st_known = false;
     std::vector<double> tck(S);
     CK(cudaMemcpy(tck.data(), ckT, sizeof(double) * S, cudaMemcpyDeviceToHost));
     // adjoint buffers
@@ -2522,6 +2531,7 @@ int adjoint_T(bm_ctx *c, int steps, int k, const double *target, int m0_scales, 
     CK(cudaMemcpy(m.buf[0], Mfin, v3, cudaMemcpyDeviceToDevice));
     c->host_st = st_end;
     CK(cudaMemcpy(c->st, &c->host_st, sizeof(StepState), cudaMemcpyHostToDevice));
+    c->st_known = true;
     c->s1_dirty = true;
     (void)st0;
     return 0;
@@ -2888,7 +2898,9 @@ int bm_set_m(bm_ctx *c, int mesh, const double *M)
     c->host_st.error = 0;   // a new M clears a non-finite state
     c->es_reset = true;
     c->dt = c->host_st.dT;
-    return upload_state(c);
+    if (int rc = upload_state(c)) return rc;
+    CK(cudaStreamSynchronize(c->stream));   // M may change once this returns
+    return 0;
 }
 
 int bm_get_m(bm_ctx *c, int mesh, double *M)
@@ -3057,7 +3069,9 @@ int bm_set_m_device(bm_ctx *c, int mesh, const void *M, int elem_bytes, void *st
     c->host_st.error = 0;
     c->es_reset = true;
     c->dt = c->host_st.dT;
-    return upload_state(c);
+    if ((rc = upload_state(c))) return rc;
+    CK(cudaStreamSynchronize(c->stream));   // M may change once this returns
+    return 0;
 }
 
 int bm_get_m_device(bm_ctx *c, int mesh, void *M, int elem_bytes, void *stream)
@@ -3117,6 +3131,7 @@ static int get_diag(bm_ctx *c, int which, double *v)
     cudaSetDevice(c->device);
     double val = 0.0;
     static const int one = 1;
+    c->st_known = false;   // the request is set in the device's copy
     const double *src = which ? &c->st->dmdt : &c->st->mxh;
     int *flag = which ? &c->st->calc_dmdt : &c->st->calc_mxh;
     CK(cudaMemcpyAsync(&val, src, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -3201,6 +3216,7 @@ namespace {
 template <typename T>
 int time_step_T(bm_ctx *c, int steps, double *ms6, double *bytes6, int *launches6)
 {
+    c->st_known = false;
     for (int k = 0; k < BM_TK_COUNT; k++) { ms6[k] = 0.0; bytes6[k] = 0.0; launches6[k] = 0; }
     if (c->batched && c->meshes.size() > 1) return fail(BM_EUNSUPPORTED, "bm_time_step: batched meshes are timed per step only");
     if (c->ml) return fail(BM_EUNSUPPORTED, "bm_time_step: the multilayered convolution has bm_ml_time_kernels");
@@ -3239,6 +3255,7 @@ int time_step_T(bm_ctx *c, int steps, double *ms6, double *bytes6, int *launches
 template <typename T>
 int time_kernels_T(bm_ctx *c, Mesh &m, int reps, double *ms4, double *bytes4)
 {
+    c->st_known = false;
     for (int i = 0; i < 4; i++) { ms4[i] = 0.0; bytes4[i] = 0.0; }
     if (m.ml_role) return fail(BM_EUNSUPPORTED, "per-mesh kernel timing of a multilayer mesh");
     cudaStream_t s = c->stream;
@@ -3318,6 +3335,7 @@ namespace {
 template <typename T>
 int ml_time_T(bm_ctx *c, int reps, double *ms6, double *bytes6)
 {
+    c->st_known = false;
     MLRun &r = *c->ml;
     const MLGeom &g = r.g;
     cudaStream_t s = c->stream;
