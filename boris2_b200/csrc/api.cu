@@ -555,10 +555,10 @@ float time_launches(cudaStream_t s, F launch, int reps)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     ms /= reps;
-    if (ms < 0.05f) {
+    if (ms < 0.012f) {
         // launches of a few microseconds: a longer run, the better of the two (3 launches alone picked
         // stage shapes twice as slow as the best on small films)
-        const int more = 4 * reps;
+        const int more = 2 * reps;
         cudaEventRecord(e0, s);
         for (int r = 0; r < more; r++) launch();
         cudaEventRecord(e1, s);
