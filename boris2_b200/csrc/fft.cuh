@@ -79,12 +79,19 @@ template <typename T, bool INV> BM_HD cpx<T> rot90(cpx<T> a)   // a * (-i) forwa
     return INV ? mul_i(a) : mul_mi(a);
 }
 
+// a +- b rotated (rot90), in scalar sums: the rotation is an exchange of the parts there
+template <typename T, bool INV> BM_HD cpx<T> add_rot(cpx<T> a, cpx<T> b)
+{
+    return INV ? mk<T>(a.x - b.y, a.y + b.x) : mk<T>(a.x + b.y, a.y - b.x);
+}
+template <typename T, bool INV> BM_HD cpx<T> sub_rot(cpx<T> a, cpx<T> b) { return add_rot<T, !INV>(a, b); }
+
 template <typename T, bool INV> BM_HD void dft4(cpx<T> *v)
 {
     cpx<T> a0 = v[0] + v[2], a1 = v[0] - v[2];
-    cpx<T> b0 = v[1] + v[3], b1 = rot90<T, INV>(v[1] - v[3]);
+    cpx<T> b0 = v[1] + v[3], d = v[1] - v[3];
     v[0] = a0 + b0; v[2] = a0 - b0;
-    v[1] = a1 + b1; v[3] = a1 - b1;
+    v[1] = add_rot<T, INV>(a1, d); v[3] = sub_rot<T, INV>(a1, d);
 }
 
 template <typename T, bool INV> BM_HD void dft8(cpx<T> *v)
@@ -97,11 +104,10 @@ template <typename T, bool INV> BM_HD void dft8(cpx<T> *v)
     dft4<T, INV>(o);
     // w^1 = s(1 -+ i), w^2 = -+i, w^3 = s(-1 -+ i)
     cpx<T> o1 = INV ? mk<T>(s * (o[1].x - o[1].y), s * (o[1].x + o[1].y)) : mk<T>(s * (o[1].x + o[1].y), s * (o[1].y - o[1].x));
-    cpx<T> o2 = rot90<T, INV>(o[2]);
     cpx<T> o3 = INV ? mk<T>(-s * (o[3].x + o[3].y), s * (o[3].x - o[3].y)) : mk<T>(s * (o[3].y - o[3].x), -s * (o[3].x + o[3].y));
     v[0] = e[0] + o[0]; v[4] = e[0] - o[0];
     v[1] = e[1] + o1;   v[5] = e[1] - o1;
-    v[2] = e[2] + o2;   v[6] = e[2] - o2;
+    v[2] = add_rot<T, INV>(e[2], o[2]); v[6] = sub_rot<T, INV>(e[2], o[2]);
     v[3] = e[3] + o3;   v[7] = e[3] - o3;
 }
 
