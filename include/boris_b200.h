@@ -344,9 +344,10 @@ int bm_time_demag(bm_ctx *ctx, int mesh, int reps, double *ms);
  * when the 3D y passes use the radix-16 Stockham transform, plus 200 when they are the persistent
  * kernels fed by pipelined bulk tensor copies),
  * z-pass width (plus 1000 when the fused y -> z -> y cluster pass replaces the three 3D passes,
- * plus 10000 when the z pass is the parity split: two threads per pencil line), stage rows per block (plus 100 when the stage kernel uses the radix-8
+ * plus 10000 when the z pass is the parity split, two threads per pencil line, 20000 when it is the FP32
+ * column pairs, two lines per thread), stage rows per block (plus 100 when the stage kernel uses the radix-8
  * Stockham x transform, 200 the radix-16 one, 300 the radix-16 one at the lower FP32 register
- * cap; negative when it prefetches its per-cell rows into shared memory)]. Valid after the first
+ * cap, 400 the FP32 butterfly pairs; negative when it prefetches its per-cell rows into shared memory)]. Valid after the first
  * compute or run. */
 int bm_tiles(bm_ctx *ctx, int mesh, int *tiles4);
 
