@@ -7,6 +7,8 @@
 // addresses and issue slots per cell. Boundary cells take the interior stencil with the missing neighbour
 // replaced by its Neumann ghost value m -+ h bd (the one-sided differences of axis_stencil are this
 // substitution), so no second copy of the stencil is needed and lanes at the x ends do not diverge.
+// Measured (stage launch of the 512 x 512 x 16 film, radix-16 x transforms): 198 -> 188 us in FP32, 407 -> 366 us in
+// FP64; 128 x 64 film 15.2 -> 13.4 us.
 //
 // ODD: nx may be odd, so rows start on any value (pairs are read and written as two scalars) and the last
 // pair of a row may have one cell: its second lane repeats the first and is never stored (zero in the x line).
