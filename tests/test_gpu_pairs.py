@@ -9,6 +9,7 @@ import pytest
 from oracle_libs import orc_hdemag, sphere_random, OracleSolver
 
 pytestmark = pytest.mark.gpu
+MU0 = 1.256637061435916e-6
 
 
 @pytest.mark.parametrize("nx", [1, 2, 3, 16, 31, 190, 257])
@@ -89,3 +90,54 @@ def test_zpair_hdemag(bm, monkeypatch, n, W):
         H = c.demag_field()
         assert c.tiles()["zmid_zv"] == 2 and c.tiles()["zmid_W"] == W
     assert np.abs(H - Href).max() / np.abs(Href).max() < 1e-5
+
+
+@pytest.mark.parametrize("n", [(64, 5, 3), (33, 4, 3), (1, 6, 4), (2, 2, 2), (50, 1, 1), (7, 9, 1)])
+@pytest.mark.parametrize("pbc", [(0, 0, 0), (1, 0, -1)])
+@pytest.mark.parametrize("D", [0.0, 5e-6])
+def test_stage_pairs_smooth_state(bm, n, pbc, D):
+    """FP32 exchange / iDMI of a state that varies little from cell to cell, at every cell, the boundaries
+    included. Differences of neighbours are exact there, so the error is bounded by the roundings after them:
+    at most 20 (the boundary term 4, 1 / h^2, the sums over sides and axes 4, the coefficient 7, its product
+    and the sum into H 2, the gradient's factors 2), each 2^-24 of the terms. A stencil that rounds a sum of two
+    neighbours first is off by 2^-24 of M instead, a thousand times the differences here."""
+    h, Ms, A = (4e-9, 3e-9, 2e-9), 8e5, 1.3e-11
+    z, y, x = np.meshgrid(*[(np.arange(k) + 0.5) / k for k in n[::-1]], indexing="ij")
+    th, ph = 0.9 + 3e-3 * np.cos(2 * x + y) + 2e-3 * z, 0.7 + 4e-3 * np.sin(x - 2 * y) - 2e-3 * z
+    M = (Ms * np.stack([np.sin(th) * np.cos(ph), np.sin(th) * np.sin(ph), np.cos(th)], -1)).astype(np.float32).astype(np.float64)
+    # terms of the stencil per cell: |neighbour - cell| per side, |h bd| at an open side
+    rr = D / (2 * A)
+    bd = {0: np.stack([rr * M[..., 2], 0 * M[..., 0], -rr * M[..., 0]], -1), 1: np.stack([0 * M[..., 0], rr * M[..., 2], -rr * M[..., 1]], -1),
+          2: 0 * M}
+    terms, grad = np.zeros_like(M), {}
+    for k, ax in ((0, 2), (1, 1), (2, 0)):
+        if n[k] == 1:
+            continue
+        d = np.abs(np.diff(M, axis=ax))
+        lo, hi = [np.abs(h[k] * np.take(bd[k], [i], axis=ax)) for i in (0, -1)]
+        if pbc[k]:
+            wrap = np.abs(pbc[k] * np.take(M, [-1], axis=ax) - np.take(M, [0], axis=ax))
+            lo = hi = wrap
+        t = np.concatenate([lo, d], axis=ax) + np.concatenate([d, hi], axis=ax)
+        terms += 2 * A / (MU0 * Ms * Ms) * t / h[k] ** 2
+        grad[k] = D / (MU0 * Ms * Ms) * t / h[k]
+    if 0 in grad:
+        terms[..., 0] += grad[0][..., 2]
+        terms[..., 2] += grad[0][..., 0]
+    if 1 in grad:
+        terms[..., 1] += grad[1][..., 2]
+        terms[..., 2] += grad[1][..., 1]
+    d = dict(n=n, h=h, Ms=Ms, A=A, D=D, modules=4 if D else 2, pbc=pbc)
+    s = OracleSolver([d])
+    s.set_m(M.reshape(-1, 3))
+    Href = s.heff()
+    s.close()
+    with bm.Context(precision=bm.MIXED) as c:
+        c.add_mesh(n, h)
+        c.set_material(0, Ms=Ms, A=A, D=D, alpha=0.1)
+        c.set_modules(0, d["modules"])
+        c.set_pbc(0, pbc)
+        c.set_m(M.reshape(-1, 3))
+        H = c.update_field()
+    bound = 20 * 2.0 ** -24 * terms.reshape(-1, 3) + 1e-9   # A/m; M and H are of the order of 1e5
+    assert (np.abs(H - Href) <= bound).all()
