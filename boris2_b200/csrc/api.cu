@@ -523,8 +523,9 @@ int upload_state(bm_ctx *c)
     return 0;
 }
 
-// the device's step state in host_st. Only the steps and the calls that request a diagnostic change it, so between
-// them (bm_set_m, bm_set_ode, the statistics after a run) the copy at hand is current and no wait is needed
+// the device's step state in host_st. Between the launches that can change it (steps, the calls that request a
+// diagnostic, and the pipelined y passes, which set its error flag when a wait gives up: yz_args) the copy at hand
+// is current and no wait is needed
 int read_state(bm_ctx *c)
 {
     if (c->st_known) return 0;
@@ -1233,6 +1234,7 @@ YZArgs<T> yz_args(bm_ctx *c, Mesh &m, int gate)
     a.pdl = c->pdl;
     a.yv = m.yv;
     a.zv = m.zv;
+    if (m.yv == 2) c->st_known = false;
     return a;
 }
 
@@ -2245,6 +2247,12 @@ int build_graph(bm_ctx *c)
     return 0;
 }
 
+int check_wait(bm_ctx *c)
+{
+    if (c->host_st.error & BM_ERR_WAIT) return fail(BM_ECUDA, "a kernel's bounded wait for its bulk tensor copies gave up");
+    return 0;
+}
+
 template <typename T>
 int run_T(bm_ctx *c, int steps)
 {
@@ -2279,8 +2287,7 @@ int run_T(bm_ctx *c, int steps)
         for (long long i = warm; i < k; i++) CK(cudaGraphLaunch(c->gexec_es, c->stream));
         guard += k;
         if ((rc = read_state(c))) return rc;
-        if (c->host_st.error & BM_ERR_WAIT)
-            return fail(BM_ECUDA, "a kernel's bounded wait for its bulk tensor copies gave up");
+        if ((rc = check_wait(c))) return rc;
         if (c->host_st.error & BM_ERR_NONFINITE)
             return fail(BM_ENONFINITE, c->eval == BM_RK4
                                            ? "a step produced a non-finite M (NaN or infinity); its steps are counted"
@@ -2289,6 +2296,18 @@ int run_T(bm_ctx *c, int steps)
         if (guard > 100LL * steps + 1000) return fail(BM_ESTATE, "step control did not converge");
     }
     return 0;
+}
+
+// the end of a single field evaluation: waits for the stream and, where a launch can have set the error flag, reads
+// the step state with the same wait and reports it (the flag stays set until a new M, as after a run)
+int finish_field(bm_ctx *c)
+{
+    if (c->st_known) {
+        CK(cudaStreamSynchronize(c->stream));
+        return 0;
+    }
+    if (int rc = read_state(c)) return rc;
+    return check_wait(c);
 }
 
 // Single field evaluations launch their kernels one by one: the programmatic dependence hides the launch
@@ -2338,9 +2357,8 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
     CKL(launch_stage<T>(a, c->stream), "heff");
     CKL(launch_planes_to_aos<T>(m.stage64, (const T *)m.Hout, m.n, c->stream), "planes_to_aos");
     CK(cudaMemcpyAsync(H, m.stage64, sizeof(double) * 3 * m.n, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     c->s1_dirty = true;
-    return 0;
+    return finish_field(c);
 }
 
 // ------------------------------------------------------------------ discrete adjoint of RK4
@@ -2549,6 +2567,16 @@ int check_mesh(bm_ctx *c, int mesh)
 
 // error text for entry points defined in other translation units
 int bm_set_error(int code, const std::string &msg) { return fail(code, msg); }
+
+// sets the device's error flag as a pipelined y pass does when its wait gives up, for tests of how it is reported
+// (no wait has to run out); the host's copy of the state does not see it
+extern "C" int bm_test_raise_wait(bm_ctx *c)
+{
+    static const int bits = BM_ERR_WAIT;
+    CK(cudaMemcpyAsync(&c->st->error, &bits, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return 0;
+}
 
 // =============================================================================== C ABI
 extern "C" {
@@ -3006,9 +3034,8 @@ int demag_device_T(bm_ctx *c, Mesh &m, const S *M, S *H, int add, double *energy
         CK(cudaStreamSynchronize(s));
         *energy = -BM_MU0 * d / (2.0 * (double)m.n);
     }
-    CK(cudaStreamSynchronize(s));
     c->s1_dirty = true;
-    return 0;
+    return finish_field(c);
 }
 
 template <typename T>

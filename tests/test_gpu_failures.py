@@ -3,6 +3,7 @@
   * a NaN planted in M by bm_set_m, and a state driven to overflow by an applied field of 1e300 A/m:
     bm_run returns BM_ENONFINITE; under RKDP54 the step is not accepted even when dT cannot shrink
     (dT_min = dT); the flag stays until a new M is set, after which the context runs normally
+  * the flag of a wait that gave up: reported by field evaluations and runs, kept until a new M is set
   * a device-memory limit below what the meshes need: set-up refuses with BM_ENOMEM before
     allocating, and the same context works once the limit is raised
 """
@@ -84,4 +85,30 @@ def test_memory_limit_refuses_before_allocating(bm):
     c.set_memory_limit(0)
     H = c.demag_field()
     assert np.isfinite(H).all() and np.abs(H).max() > 0
+    c.close()
+
+
+def test_failed_wait_is_reported_and_kept(bm, monkeypatch):
+    """The error flag that a pipelined y pass sets when its bounded wait gives up (set from the host here, no wait
+    runs out): a field evaluation with such passes reports it, a change of step parameters does not lose it, the
+    next run reports it too, and a new M clears it."""
+    monkeypatch.setenv("BM_TILES", "2,8,8,1")
+    monkeypatch.setenv("BM_Y_XV", "2")
+    c = _film(bm, bm.MIXED, "RK4")
+    M = sphere_random(NC, seed=5, Ms=8e5)
+    for parameters in (lambda: c.setdt(1e-13), lambda: c.astepctrl(1e-5, 2.0, 1e-15, 3e-12)):
+        c.set_m(M)
+        H = c.demag_field()
+        assert c.tiles()["ypass_yv"] == 2
+        assert bm.lib().bm_test_raise_wait(c._h) == 0
+        with pytest.raises(bm.BorisError) as e:
+            c.demag_field()
+        assert e.value.code == bm.ECUDA and "wait" in str(e.value)
+        parameters()
+        with pytest.raises(bm.BorisError) as e:
+            c.run(2)
+        assert e.value.code == bm.ECUDA and "wait" in str(e.value)
+        c.set_m(M)
+        assert np.array_equal(c.demag_field(), H)
+        c.run(2)
     c.close()
