@@ -1,7 +1,7 @@
 """Kernels that carry two x-adjacent values per thread, on cuda:0 against the oracle: the stage kernel's
 per-cell part on cell pairs (even and odd nx down to 1, every field term, open and periodic, each x
-transform variant, the FP32 x transforms on butterfly pairs) and the FP32 z pass on column pairs (BM_Z_XV=2;
-each length, partial tiles).
+transform variant at lengths that have it, the FP32 x transforms on butterfly pairs) and the FP32 z pass on
+column pairs (BM_Z_XV=2; each length, partial tiles).
 Bounds as elsewhere: FP64 1e-9 and mixed 1e-5 of the largest field, states FP64 1e-9, mixed 1e-4 of Ms."""
 import numpy as np
 import pytest
@@ -12,9 +12,14 @@ pytestmark = pytest.mark.gpu
 MU0 = 1.256637061435916e-6
 
 
-@pytest.mark.parametrize("nx", [1, 2, 3, 16, 31, 190, 257])
+# (x-transform variant, nx): every nx has the two-level / generic form; Stockham from 16 packed elements, radix 16
+# at 256, 512 and 1024 of them
+XV_NX = [("0", n) for n in (1, 2, 3, 16, 31, 190, 257)] + [("1", n) for n in (16, 31, 190, 257)] + \
+        [("2", n) for n in (201, 256, 401, 512)]
+
+
+@pytest.mark.parametrize("xv,nx", XV_NX)
 @pytest.mark.parametrize("pbc", [(0, 0, 0), (2, -1, 1)])
-@pytest.mark.parametrize("xv", ["0", "1", "2"])
 @pytest.mark.parametrize("prec,tol", [("fp64", 1e-9), ("mixed", 1e-4)])
 def test_stage_pairs(bm, monkeypatch, nx, pbc, xv, prec, tol):
     monkeypatch.setenv("BM_TILES", "1,1,4,2")
@@ -38,6 +43,7 @@ def test_stage_pairs(bm, monkeypatch, nx, pbc, xv, prec, tol):
                 c.astepctrl(1e-4, 2.0, 2e-14, 2e-14)
             c.set_m(M)
             H, Href = c.update_field(), s.heff()
+            assert c.tiles()["stage_xv"] == int(xv)
             assert np.abs(H - Href).max() / np.abs(Href).max() < (1e-9 if prec == "fp64" else 1e-5)
             c.run(6)
             s.run(6)
@@ -47,26 +53,39 @@ def test_stage_pairs(bm, monkeypatch, nx, pbc, xv, prec, tol):
 
 @pytest.mark.parametrize("nx", [49, 64, 100, 128, 201, 256, 401, 512, 1000])
 @pytest.mark.parametrize("rows", [1, 3])
-def test_stage_butterfly_pairs(bm, monkeypatch, nx, rows):
-    """The FP32 x transforms on butterfly pairs (BM_STAGE_XV=4): field, RK4 and RKDP54 steps."""
+@pytest.mark.parametrize("pbc", [(0, 0, 0), (2, -1, 1)])
+def test_stage_butterfly_pairs(bm, monkeypatch, nx, rows, pbc):
+    """The FP32 x transforms on butterfly pairs (BM_STAGE_XV=4), open and periodic, uniform and with Ms / K1 maps
+    (three rows): field, RK4 and RKDP54 steps."""
     monkeypatch.setenv("BM_TILES", "1,1,4,%d" % (rows if nx < 600 else min(rows, 2)))
     monkeypatch.setenv("BM_STAGE_XV", "4")
     d = dict(n=(nx, 3, 2), h=(4e-9, 3e-9, 2e-9), Ms=8e5, A=1.3e-11, D=1.5e-3, alpha=0.1, K1=1e5, modules=1 | 4 | 8 | 16,
-             Ha=(2e4, -1e4, 5e3))
+             Ha=(2e4, -1e4, 5e3), pbc=pbc)
     M = sphere_random(int(np.prod(d["n"])), seed=9 + nx, Ms=8e5)
+    if rows == 3:
+        rng = np.random.default_rng(nx)
+        d["Ms_map"] = 8e5 * rng.uniform(0.9, 1.1, len(M))
+        d["K1_map"] = 1e5 * rng.uniform(0.5, 1.5, len(M))
+        M *= d["Ms_map"][:, None] / 8e5
     for ode in (0, 1):
         s = OracleSolver([d], evaluation=ode, dt=2e-14, dT_min=2e-14, dT_max=2e-14)
         s.set_m(M)
         with bm.Context(precision=bm.MIXED) as c:
             c.add_mesh(d["n"], d["h"])
             c.set_material(0, Ms=d["Ms"], A=d["A"], alpha=d["alpha"], K1=d["K1"], D=d["D"])
+            if rows == 3:
+                c.set_material_maps(0, Ms_map=d["Ms_map"], K1_map=d["K1_map"])
             c.set_modules(0, d["modules"])
+            c.set_pbc(0, pbc)
             c.set_field(0, d["Ha"])
             c.setode("RKDP54" if ode else "RK4", 2e-14)
             if ode:
                 c.astepctrl(1e-4, 2.0, 2e-14, 2e-14)
             c.set_m(M)
-            H, Href = c.demag_field(), orc_hdemag(M, d["n"], d["h"])[0]
+            if not any(pbc):
+                H, Href = c.demag_field(), orc_hdemag(M, d["n"], d["h"])[0]
+                assert np.abs(H - Href).max() / np.abs(Href).max() < 1e-5
+            H, Href = c.update_field(), s.heff()
             assert c.tiles()["stage_xv"] == 4
             assert np.abs(H - Href).max() / np.abs(Href).max() < 1e-5
             c.run(6)
