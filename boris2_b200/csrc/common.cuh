@@ -13,7 +13,7 @@ template <typename T> using cpx = cpx_t<T>;
 template <typename T> BM_HD cpx<T> mk(T a, T b) { cpx<T> r; r.x = a; r.y = b; return r; }
 template <typename T> BM_HD cpx<T> operator+(cpx<T> a, cpx<T> b) { return mk<T>(a.x + b.x, a.y + b.y); }
 template <typename T> BM_HD cpx<T> operator-(cpx<T> a, cpx<T> b) { return mk<T>(a.x - b.x, a.y - b.y); }
-#ifdef __CUDA_ARCH__
+#if defined(__CUDA_ARCH__) && !defined(BM_SCALAR_SUMS)
 // FP32 sums and differences of complex values as one packed instruction (each lane rounded as its scalar form):
 // most of a register FFT's arithmetic, at half the issue slots. On the 512 x 512 x 16 film the z pass went 150 ->
 // 139 us and the y passes 92.8 / 99.2 -> 88.3 / 92.2.

@@ -1476,19 +1476,11 @@ static int ypass_reg_batch_dispatch(int Ny, const YZArgs<T> *dargs, const int2 *
     case 8: return launch_ypass_reg_batch<T, 8, INV>(dargs, dwork, nwork, nt, smem, s);
     case 16: return launch_ypass_reg_batch<T, 16, INV>(dargs, dwork, nwork, nt, smem, s);
     case 32: return launch_ypass_reg_batch<T, 32, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 64: return launch_ypass_reg_batch<T, 64, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 128: return launch_ypass_reg_batch<T, 128, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 256: return launch_ypass_reg_batch<T, 256, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 512: return launch_ypass_reg_batch<T, 512, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 1024: return launch_ypass_reg_batch<T, 1024, INV>(dargs, dwork, nwork, nt, smem, s);
     case 12: return launch_ypass_reg_batch<T, 12, INV>(dargs, dwork, nwork, nt, smem, s);
     case 24: return launch_ypass_reg_batch<T, 24, INV>(dargs, dwork, nwork, nt, smem, s);
     case 48: return launch_ypass_reg_batch<T, 48, INV>(dargs, dwork, nwork, nt, smem, s);
     case 96: return launch_ypass_reg_batch<T, 96, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 192: return launch_ypass_reg_batch<T, 192, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 384: return launch_ypass_reg_batch<T, 384, INV>(dargs, dwork, nwork, nt, smem, s);
-    case 768: return launch_ypass_reg_batch<T, 768, INV>(dargs, dwork, nwork, nt, smem, s);
-    default: return 111;
+    default: return 111;   // the longer ones: launch_ypass_long_batch
     }
 }
 
@@ -1544,10 +1536,13 @@ int launch_yz_batch(int kind, int key, const YZArgs<T> *dargs, const int2 *dwork
         case 1024: return launch_ymid2d_reg_batch<T, 1024>(dargs, dwork, nwork, nt, smem, s);
         default: return 111;
         }
-    case BM_BATCH_YFWD_ST: return ypass_st_batch_dispatch<T, false>(key, dargs, dwork, nwork, nt, smem, s);
-    case BM_BATCH_YINV_ST: return ypass_st_batch_dispatch<T, true>(key, dargs, dwork, nwork, nt, smem, s);
-    case BM_BATCH_YFWD_REG: return ypass_reg_batch_dispatch<T, false>(key, dargs, dwork, nwork, nt, smem, s);
-    case BM_BATCH_YINV_REG: return ypass_reg_batch_dispatch<T, true>(key, dargs, dwork, nwork, nt, smem, s);
+    case BM_BATCH_YFWD_ST: case BM_BATCH_YINV_ST: return launch_ypass_long_batch<T>(kind, key, dargs, dwork, nwork, nt, smem, s);
+    case BM_BATCH_YFWD_REG:
+        if (ypass_long_batch(key)) return launch_ypass_long_batch<T>(kind, key, dargs, dwork, nwork, nt, smem, s);
+        return ypass_reg_batch_dispatch<T, false>(key, dargs, dwork, nwork, nt, smem, s);
+    case BM_BATCH_YINV_REG:
+        if (ypass_long_batch(key)) return launch_ypass_long_batch<T>(kind, key, dargs, dwork, nwork, nt, smem, s);
+        return ypass_reg_batch_dispatch<T, true>(key, dargs, dwork, nwork, nt, smem, s);
     default: return 110;
     }
     return (int)cudaGetLastError();

@@ -232,6 +232,12 @@ template <typename T> int launch_stage(const StageArgs<T> &a, cudaStream_t s);
 template <typename T>
 int launch_yz_batch(int kind, int key, const YZArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem,
                     cudaStream_t s);
+// the list launches of the 3D y passes with long lines (demag_ylist.cuh): two-level of power-of-two length from 64,
+// and the Stockham ones
+constexpr bool ypass_long_batch(int Ny) { return Ny >= 64 && Ny % 3 != 0; }
+template <typename T>
+int launch_ypass_long_batch(int kind, int Ny, const YZArgs<T> *dargs, const int2 *dwork, int nwork, int nt, size_t smem,
+                            cudaStream_t s);
 // the twiddle tables of xv 4 for x length LX (host; empty where it has none)
 std::vector<float> stage_pair_tables(int LX);
 // key 0: generic-length stage kernel; key LX: the radix-8 register kernel of that length

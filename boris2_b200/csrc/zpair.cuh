@@ -180,8 +180,9 @@ template <int NZ> static int launch_zpair_n(const YZArgs<float> &a, cudaStream_t
     }
 }
 
-// the z pass on column pairs, or -1 where it does not apply (zmid_has_pair)
-static int launch_zmid_pair(const YZArgs<float> &a, cudaStream_t s)
+// the z pass on column pairs, or -1 where it does not apply (zmid_has_pair); a template, so that only the z pass'
+// translation unit holds its kernels
+template <typename T> static int launch_zmid_pair(const YZArgs<T> &a, cudaStream_t s)
 {
     if (!zmid_has_pair(a.Nz, a.W, a.LX)) return -1;
     switch (a.Nz) {

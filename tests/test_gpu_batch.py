@@ -114,3 +114,23 @@ def test_batched_wide_systems_equal_per_mesh(bm):
         c.close()
     err = max(np.abs(a - b).max() / d["Ms"] for a, b, d in zip(out[0], out[1], descs))
     assert err < 1e-11
+
+
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-9), ("mixed", 1e-4)])
+def test_batched_y_lengths(bm, prec, tol):
+    """Work-list y passes of every kind: two-level lines of 8 to 1024 points (from 64 on in their own translation
+    unit), 3 * 2^k ones, Stockham and generic ones, against the oracle."""
+    ny = [3, 7, 16, 31, 50, 128, 200, 400, 5, 12, 20, 40, 90, 150, 350, 700, 1000]
+    descs = [dict(n=(9, n, 2), h=H, Ms=8e5, A=1.3e-11, alpha=0.2, modules=1 | 2) for n in ny]
+    M0 = _init(descs, "sphere")
+    s = OracleSolver(descs, evaluation=0, dt=5e-14)
+    c = _ctx(bm, prec, True, descs, "RK4", 5e-14)
+    for q, M in enumerate(M0):
+        s.set_m(M, q)
+        c.set_m(M, q)
+    s.run(3)
+    c.run(3)
+    err = [np.abs(c.get_m(q) - s.get_m(q)).max() / d["Ms"] for q, d in enumerate(descs)]
+    c.close()
+    s.close()
+    assert max(err) < tol, dict(zip(ny, err))
