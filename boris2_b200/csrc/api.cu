@@ -377,20 +377,45 @@ void choose_tiles(Mesh &m)
 // Meshes of a batch large enough to fill the GPU by themselves get launches of their own, as parallel branches
 // beside the work-list launches of the small ones: a work-list kernel reads its arguments from memory, takes
 // the block shape of the largest mesh of its group, and has no column-pair or butterfly-pair form.
+// The line, RK4 step of 4 / 16 / 64 equal meshes with own launches over work lists: (64,64,8), 32768 cells, 0.73 /
+// 0.75 / 0.86; (256,128,1) 0.80 / 1.03 / 0.98; (192,192,1) 0.72 / 0.67 / 0.64; (256,256,1) 0.74 / 0.69 / 0.73; below,
+// (128,128,1) 0.79 / 1.21 / 1.15, (96,96,2) 0.91 / 1.12 / 1.26, (64,200,2) 0.75 / 0.69 / 0.73, FP64 0.69 .. 0.94.
+// A 2D length without a register y pass (Ny 1536 and from 2048) runs the generic kernel either way and gains
+// nothing: (80,700,1) 1.06 / 1.11 / 0.92 for 2 / 4 / 16 meshes, FP64 1.10 / 1.21 / 1.16.
 constexpr long long kSoloCells = 32768;
-bool batch_solo(const Mesh &m) { return m.n >= kSoloCells; }
+bool batch_solo(int nx, int ny, int nz)
+{
+    return (long long)nx * ny * nz >= kSoloCells && (nz > 1 || ypass_has_reg(2 * nice_size(ny)));
+}
 
-// tile shapes of a batch's large meshes without timing (a batch has hundreds of meshes to set up)
+// tile shapes of a batch's large meshes without timing (a batch has hundreds of meshes to set up). Block shapes
+// of the stage kernel: FP32 films take 192 threads (16 x (256,128,1): step 225 us, 251 with 96), the rest 96 and at
+// least two blocks per SM (16 x (64,64,8) in FP64 453 us, 500 with 192; 4 of them in FP32 112 us, 119). Four columns
+// per block in the 2D y pass: within 3 % of eight, and two cost up to 19 % (16 x (300,120,1) 313 -> 373 us).
 template <typename T> void solo_tiles(Mesh &m)
 {
     const bool f = sizeof(T) == 4;
     m.xv = f && stage_reg_q(m.LX, 4) ? 4 : stage_reg_q(m.LX, 2) ? 2 : stage_reg_q(m.LX, 1) ? 1 : 0;
     const int tpl = stage_reg_q(m.LX, m.xv) ? stage_reg_q(m.LX, m.xv) : m.px.tpl, rows = m.ny * m.nz;
-    m.rpb = std::max(1, std::min(96 / (3 * tpl), rows / 296));
+    if (f && m.nz == 1) m.rpb = std::max(1, std::min(192 / (3 * tpl), rows / 37));
+    else m.rpb = std::max(1, std::min(96 / (3 * tpl), rows / 296));
     if (m.nz == 1) {
         m.W2 = 4;
-        while (m.W2 > 1 && (ymid2d_smem<T>(m.Ny, m.W2) > 110 * 1024 || m.W2 > m.LX || 3 * m.W2 * m.py.tpl > bm_lb<T>::v)) m.W2 /= 2;
-    } else if (f && m.Nz <= 16 && zmid_has_pair(m.Nz, 32, m.LX)) {
+        while (m.W2 > 1 && (ymid2d_smem<T>(m.Ny, m.W2) > 110 * 1024 || m.W2 > m.LX || ymid2d_reg_threads(m.Ny, m.W2) > bm_lb<T>::v))
+            m.W2 /= 2;
+        return;
+    }
+    // lengths without a two-level y pass: the Stockham one (16 x (40,1000,2) step 1143 us, generic kernel 1213; FP64
+    // 1962 / 2003)
+    if (ypass_has_st(m.Ny) && !ypass_has_reg(m.Ny)) {
+        int W = 16;
+        while (W > 2 && (ypass_st_threads(m.Ny, W) > 256 || (size_t)m.Ny * W * sizeof(cpx<T>) > 64 * 1024 || W > m.LX)) W /= 2;
+        if (ypass_st_threads(m.Ny, W) % 32 == 0) {
+            m.yv = 1;
+            m.Wy = W;
+        }
+    }
+    if (f && m.Nz <= 16 && zmid_has_pair(m.Nz, 32, m.LX)) {
         m.zv = 2;
         m.Wz = 32;
     } else {
@@ -574,8 +599,6 @@ float time_launches(cudaStream_t s, F launch, int reps)
     return ms;
 }
 
-// Row counts per block the stage tuner tries: 1, and more while at least one block per SM remains (fewer
-// blocks only leave SMs idle: 7 blocks of 480 threads took 21 us where 64 blocks of one row took 10)
 template <typename T> bool tune_xv_ok(int LX, int xv)
 {
     // x-transform variants a length has: 0 always (the generic kernel where there is no register one), 3 (radix
@@ -585,6 +608,8 @@ template <typename T> bool tune_xv_ok(int LX, int xv)
     if (xv == 3 && stage_reg_q(LX, 4)) return false;   // the pairs are faster wherever the lower cap was
     return stage_reg_q(LX, xv) != 0 && (xv == 2 || sizeof(T) == 4);
 }
+// Row counts per block the stage tuner tries: 1, and more while at least one block per SM remains (fewer
+// blocks only leave SMs idle: 7 blocks of 480 threads took 21 us where 64 blocks of one row took 10)
 bool tune_rows_ok(int rows, int rpb) { return rpb == 1 || (rows + rpb - 1) / rpb >= 148; }
 
 // 3D y passes of one grid: transform variant (two-level register / radix-16 Stockham) x column
@@ -1089,7 +1114,7 @@ int prepare_T(bm_ctx *c)
             if (sz && sz[0] == '1' && m.nz > 1 && m.ml_role == 0 && (m.modules & BM_DEMAG) && !c->batched)
                 m.yzy = yzy_available<T>(yz_args<T>(c, m, BM_GATE_ALWAYS)) == 0 ? 1 : 0;
         } else if (c->batched) {
-            if (batch_solo(m)) solo_tiles<T>(m);
+            if (batch_solo(m.nx, m.ny, m.nz)) solo_tiles<T>(m);
         } else if (c->autotune) {
             autotune_mesh<T>(c, m);
         }
@@ -1310,7 +1335,9 @@ template <typename T> T *E(Mesh &m, int i) { return (T *)m.ev[i]; }
 // context to another side stream that waits for the fork point, join() brings the work back to the main
 // stream. The launches of one pass of a batch (one per transform length) touch different meshes, and most
 // of them fill a fraction of the GPU (48 .. 180 blocks), so one after another they leave it idle: 24 uneven
-// films took 3.13 ms of summed kernel time per RK4 step.
+// films took 3.13 ms of summed kernel time per RK4 step. 15 side streams: with 7 the launches of many small meshes
+// queued behind one another (16 films of 256 x 128 cells 249 us a step with 15, 304 with 7, 408 with 3, 218 in work
+// lists; 31 streams change no case by more than 7 % either way).
 struct Branches {
     bm_ctx *c;
     cudaStream_t main;
@@ -1361,7 +1388,7 @@ struct Branches {
     }
     // an error path leaves the context on its own stream
     ~Branches() { c->stream = main; }
-    static constexpr int kSide = 7;
+    static constexpr int kSide = 15;
 };
 
 // ------------------------------------------------------------------ many meshes per launch
@@ -1373,11 +1400,9 @@ size_t bp_append(BatchPlan &bp, const void *p, size_t bytes)
     return off;
 }
 
-// stage kernels of several meshes: per-mesh launches, or one launch over (mesh, row block) items
-// with the generic-length kernel (rows per block chosen so every mesh fills ~256 threads)
-// stage kernels of every mesh: one launch per x length with a radix-8 register kernel, one for
-// the remaining lengths (generic kernel), as parallel branches. The last work item of the set's launches
-// finishes the step (error-norm controller, time advance).
+// stage kernels of a batch: own launches of the large meshes, one launch over (mesh, row block) items per x length
+// with a register kernel and one for the remaining lengths (generic kernel), as parallel branches. The last work
+// item of the set's launches finishes the step (error-norm controller, time advance).
 template <typename T>
 int stage_batch_one(bm_ctx *c, int key, std::vector<StageArgs<T>> &v, int *count)
 {
@@ -1451,7 +1476,7 @@ int stage_multi(bm_ctx *c, std::vector<StageArgs<T>> &v, int *count)
     std::vector<StageArgs<T>> solo;
     unsigned int total = 0;   // work items of the set: the large meshes' blocks and the work lists
     for (auto &a : v) {
-        if (a.n < kSoloCells) {
+        if (!batch_solo(a.nx, a.ny, a.nz)) {
             groups[stage_reg_q(a.LX, 1) ? a.LX : 0].push_back(a);
             continue;
         }
@@ -1565,7 +1590,7 @@ int yz_multi(bm_ctx *c, int gate, int *count)
     int rc;
     for (auto &m : c->meshes) {
         if (!(m.modules & BM_DEMAG)) continue;
-        if (batch_solo(m)) {
+        if (batch_solo(m.nx, m.ny, m.nz)) {
             if ((rc = br.next())) return rc;
             if (c->bp.collect) continue;   // nothing to collect: launched with its own arguments
             if ((rc = enqueue_yz<T>(c, m, gate, count))) return rc;
