@@ -567,8 +567,10 @@ int read_state(bm_ctx *c)
 template <typename T> YZArgs<T> yz_args(bm_ctx *c, Mesh &m, int gate);
 template <typename T> StageArgs<T> stage_args(bm_ctx *c, Mesh &m);
 
+// Launches of a few microseconds that may beat the best so far get a second, longer run, the better of the two (3
+// launches alone picked stage shapes twice as slow as the best on small films); without a best one run is all.
 template <typename F>
-float time_launches(cudaStream_t s, F launch, int reps)
+float time_launches(cudaStream_t s, F launch, int reps, float best = 0.f)
 {
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
@@ -581,9 +583,7 @@ float time_launches(cudaStream_t s, F launch, int reps)
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     ms /= reps;
-    if (ms < 0.012f) {
-        // launches of a few microseconds: a longer run, the better of the two (3 launches alone picked
-        // stage shapes twice as slow as the best on small films)
+    if (ms < 0.012f && ms < 1.5f * best) {
         const int more = 2 * reps;
         cudaEventRecord(e0, s);
         for (int r = 0; r < more; r++) launch();
@@ -601,11 +601,12 @@ float time_launches(cudaStream_t s, F launch, int reps)
 
 template <typename T> bool tune_xv_ok(int LX, int xv)
 {
-    // x-transform variants a length has: 0 always (the generic kernel where there is no register one), 3 (radix
-    // 16 at the lower register cap) and 4 (butterfly pairs) in FP32
+    // x-transform variants a length has: 0 always (the generic kernel where there is no register one), 4 (butterfly
+    // pairs) in FP32. Radix 16 (2, and 3 at the lower register cap) is not timed where FP32 has the pairs: over 34
+    // shapes with LX 256 .. 1024 it was never the fastest
     if (xv == 0) return true;
     if (xv == 1) return stage_reg_q(LX, 1) != 0;
-    if (xv == 3 && stage_reg_q(LX, 4)) return false;   // the pairs are faster wherever the lower cap was
+    if (xv < 4 && sizeof(T) == 4 && stage_reg_q(LX, 4)) return false;
     return stage_reg_q(LX, xv) != 0 && (xv == 2 || sizeof(T) == 4);
 }
 // Row counts per block the stage tuner tries: 1, and more while at least one block per SM remains (fewer
@@ -686,8 +687,8 @@ int tune_grid_x(bm_ctx *c, Mesh &G)
             f.rpb = h.rpb = rpb;
             f.xv = h.xv = xv;
             f.staged = h.staged = 0;
-            float t = time_launches(s, [&]() { return launch_stage<T>(f, s); }, 3) +
-                      time_launches(s, [&]() { return launch_stage<T>(h, s); }, 3);
+            float t = time_launches(s, [&]() { return launch_stage<T>(f, s); }, 3, best) +
+                      time_launches(s, [&]() { return launch_stage<T>(h, s); }, 3, best);
             if (t < best) { best = t; br = rpb; bx = xv; }
         }
     G.rpb = br;
@@ -712,7 +713,7 @@ void tune_grid_yz(bm_ctx *c, Mesh &m)
             for (int W = 1; W <= 16 && W <= m.LX; W *= 2) {
                 if (ymid2d_smem<T>(m.Ny, W) > 200 * 1024 || W * m.py.tpl > lim) continue;
                 a.W = W;
-                float t = time_launches(s, [&]() { return launch_ymid2d<T>(a, s); }, reps);
+                float t = time_launches(s, [&]() { return launch_ymid2d<T>(a, s); }, reps, best);
                 if (t < best) { best = t; bw = W; }
             }
             m.W2 = bw;
@@ -729,7 +730,7 @@ void tune_grid_yz(bm_ctx *c, Mesh &m)
                     if (zv == 1 && !zmid_has_par(m.Nz, W)) continue;
                     if (zv == 2 && !(sizeof(T) == 4 && zmid_has_pair(m.Nz, W, m.LX))) continue;
                     a.zv = zv;
-                    float t = time_launches(s, [&]() { return launch_zmid<T>(a, s); }, reps);
+                    float t = time_launches(s, [&]() { return launch_zmid<T>(a, s); }, reps, best);
                     if (t < best) { best = t; bw = W; bzv = zv; }
                 }
             }
@@ -789,7 +790,7 @@ int autotune_mesh(bm_ctx *c, Mesh &m)
                 if ((size_t)3 * rpb * padded_len(m.LX) * cs > 200 * 1024) break;
                 a.rpb = rpb;
                 a.xv = xv;
-                float t = time_launches(s, [&]() { return launch_stage<T>(a, s); }, reps);
+                float t = time_launches(s, [&]() { return launch_stage<T>(a, s); }, reps, best);
                 if (t < best) { best = t; br = rpb; bx = xv; }
             }
         m.rpb = br;
@@ -1057,14 +1058,18 @@ int prepare_ml(bm_ctx *c)
         return 0;
     }
     r.vec = 0;
+    // where the whole-vector form applies, the line form is not timed on fewer than four columns: with two it was the
+    // fastest of all forms in none of 60 stacks, at up to 2.4 times the best line form
+    bool vec = false;
+    for (int W = 8; W <= 64 && W <= LX; W *= 2) vec = vec || zmid_ml_has_vec<T>(ml_zargs<T>(c, W, BM_GATE_ALWAYS));
     for (int W = 1; W <= 32 && W <= LX; W *= 2) {
         MLZArgs<T> z = ml_zargs<T>(c, W, BM_GATE_ALWAYS);
         z.st = nullptr;
         if (((6 * L * W + 31) & ~31) > lim || zmid_ml_smem<T>(L, g.N[2], W, z.ksm) > 200 * 1024) continue;
         if (!r.W) r.W = W;
-        if (!c->autotune) continue;
+        if (!c->autotune || (vec && W <= 2)) continue;
         z.vec = 0;
-        float t = time_launches(s, [&]() { return launch_zmid_ml<T>(z, s); }, 3);
+        float t = time_launches(s, [&]() { return launch_zmid_ml<T>(z, s); }, 3, best);
         if (t < best) { best = t; r.W = W; }
     }
     for (int W = 8; W <= 64 && W <= LX && c->autotune; W *= 2) {
@@ -1072,7 +1077,7 @@ int prepare_ml(bm_ctx *c)
         z.st = nullptr;
         z.vec = 1;
         if (!zmid_ml_has_vec<T>(z)) continue;
-        float t = time_launches(s, [&]() { return launch_zmid_ml<T>(z, s); }, 3);
+        float t = time_launches(s, [&]() { return launch_zmid_ml<T>(z, s); }, 3, best);
         if (t < best) { best = t; r.W = W; r.vec = 1; }
     }
     if (!r.W) return fail(BM_EUNSUPPORTED, "multilayer: no z-pass tile fits");
