@@ -10,7 +10,9 @@
 // A sum of two neighbours minus 2 m rounds at the size of M: relative FP32 error of the exchange field of a
 // smooth 200 x 150 film 1.0e-4 that way, 6e-8 with differences (97 x 61 x 23 box 1.1e-5, 7e-8).
 // Measured (stage launch of the 512 x 512 x 16 film, radix-16 x transforms): 198 -> 188 us in FP32, 407 -> 366 us in
-// FP64; 128 x 64 film 15.2 -> 13.4 us.
+// FP64 (380 with the stencil in differences); 128 x 64 film 15.2 -> 13.4 us. Differences taken separately for the two
+// cells, with the one between them formed once, cost FP32 nothing (168.6 us with butterfly pairs; all by pairs 171.4,
+// sums 169.2); in FP64 every form of them takes 379 to 381 us, the sums only inside too.
 //
 // ODD: nx may be odd, so rows start on any value (pairs are read and written as two scalars) and the last
 // pair of a row may have one cell: its second lane repeats the first and is never stored (zero in the x line).
@@ -180,8 +182,8 @@ __device__ __forceinline__ void stage_pairs(const StageArgs<T> &a, cpx<T> *sm, i
                 for (int c = 0; c < 3; c++) H[c] = pk_add(H[c], prow_ld<ODD>(Hd + c * n + cell, o2));
             }
             if (exch) {
-                // a missing neighbour is the far side times the axis' sign (periodic) or the ghost
-                // m -+ h bd (bd = 0 on a one-cell axis)
+                // a missing neighbour is the far side times the axis' sign (periodic) or leaves the boundary term
+                // -+ h bd (bd = 0 on a one-cell axis) in place of its difference
                 const bool px = a.pbc[0] && nx > 1, py = a.pbc[1] && ny > 1, pz = a.pbc[2] && nz > 1;
                 const bool ex0 = p == 0, ex1 = p == half - 1, ey0 = y == 0, ey1 = y == ny - 1, ez0 = z == 0, ez1 = z == nz - 1;
                 // the left neighbour of the pair's first cell, the right one of its last
@@ -205,12 +207,11 @@ __device__ __forceinline__ void stage_pairs(const StageArgs<T> &a, cpx<T> *sm, i
                     if (ey1 && py) yp = pk_mul(pk_bc<T>((T)a.pbc[1]), yp);
                     // the neighbours minus the cell; at an open side the boundary term -+ h bd instead, with h bd
                     // x (rr m2, 0, -rr m0), y (0, rr m2, -rr m1)
-                    cpx<T> dxm = pk_sub(mk<T>(xl, m[c].x), m[c]), dxp = pk_sub(mk<T>(two ? m[c].y : xr, xr), m[c]);
-                    if (ex0 && !px) dxm.x = c == 0 ? -bhx * m[2].x : c == 1 ? (T)0 : bhx * m[0].x;
-                    if (ex1 && !px) {
-                        dxp.y = c == 0 ? bhx * m[2].y : c == 1 ? (T)0 : -bhx * m[0].y;
-                        if (!two) dxp.x = dxp.y;
-                    }
+                    T dl = xl - m[c].x, dr = xr - m[c].y;
+                    const T e = m[c].y - m[c].x;   // between the two cells; zero where there is one
+                    if (ex0 && !px) dl = c == 0 ? -bhx * m[2].x : c == 1 ? (T)0 : bhx * m[0].x;
+                    if (ex1 && !px) dr = c == 0 ? bhx * m[2].y : c == 1 ? (T)0 : -bhx * m[0].y;
+                    const cpx<T> dxm = mk<T>(dl, -e), dxp = mk<T>(two ? e : dr, dr);
                     cpx<T> dym = pk_sub(ym, m[c]), dyp = pk_sub(yp, m[c]);
                     const cpx<T> b = c == 1 ? m[2] : m[1];
                     const T sb = c == 0 ? (T)0 : c == 1 ? bhy : -bhy;
