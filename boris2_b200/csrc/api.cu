@@ -176,6 +176,7 @@ struct bm_ctx {
     StepState host_st;
     bool st_known = false;     // host_st equals the device's step state (nothing that writes it has run since)
     bool batched = false;       // many meshes per launch (work lists) instead of one launch per mesh
+    int n_side = 7;             // side streams of a batched step's branches (branch_streams)
     BatchPlan bp;
     int ml_mode = -1;           // -1 off; 0 3D, 1 2D, 2 2D layered, 3 supermesh
     double sm_h[3] = {5e-9, 5e-9, 5e-9};   // requested supermesh cellsize (the reference's default h_fm)
@@ -421,6 +422,23 @@ template <typename T> void solo_tiles(Mesh &m)
     } else {
         while (m.Wz > 16) m.Wz /= 2;
     }
+}
+
+// Side streams of a batch: 15 where its large meshes are small enough that 16 of them stay in L2 between passes (with
+// 7 their launches queue behind one another), else 7 (with 15 the passes of more meshes than fit in L2 run side by
+// side). Step of 16 films of 256 x 128 cells 249 us with 15, 304 with 7, 408 with 3 (work lists 218); FP32, 15 over 7
+// streams at 24 / 64 equal meshes: 61440 cells 0.88 / 0.92, 65536 (3D) 0.90 / 0.99, 131072 (3D) 1.00 / 1.07; 256
+// films of 64 .. 512 cells a side and 1 .. 4 layers 16.1 ms against 14.9. FP64 at 16 / 64: 32768 cells 0.78 / 0.86,
+// 40000 0.86 / 0.94, 65536 (3D) 0.98 / 1.09.
+template <typename T> int branch_streams(const std::vector<Mesh> &meshes)
+{
+    long long cells = 0, large = 0;
+    for (auto &m : meshes)
+        if (batch_solo(m.nx, m.ny, m.nz)) {
+            cells += (long long)m.nx * m.ny * m.nz;
+            large++;
+        }
+    return large && cells <= large * (sizeof(T) == 4 ? 65536 : 40960) ? 15 : 7;
 }
 
 template <typename T>
@@ -779,8 +797,8 @@ int autotune_mesh(bm_ctx *c, Mesh &m)
         a.Mout = tmp + 3 * m.n;
         float best = 1e30f; int br = m.rpb, bx = 0;
         int rows = m.ny * m.nz;
-        // x-transform variant x rows per block (rows staged in shared memory are not tried: with cells in
-        // pairs they are slower at every size, 256 x 256 x 4 cells 46 against 27 us)
+        // x-transform variant x rows per block (rows staged in shared memory are not tried: with cells in pairs
+        // they are slower at each of ten sizes, stage launch FP32 1.21 to 1.73 times, FP64 1.02 to 1.78 times)
         a.staged = 0;
         for (int xv = 0; xv <= 4; xv++)
             for (int rpb = 1; rpb <= 16 && rpb <= rows; rpb++) {
@@ -1090,6 +1108,7 @@ template <typename T>
 int prepare_T(bm_ctx *c)
 {
     if (int rc = ml_plan(c)) { free_ml(c); for (auto &mm : c->meshes) mm.ml_role = 0; return rc; }
+    c->n_side = branch_streams<T>(c->meshes);
     for (auto &m : c->meshes) {
         int rc = prepare_mesh<T>(c, m);
         if (rc) { for (auto &mm : c->meshes) free_mesh(mm); free_ml(c); return rc; }
@@ -1340,9 +1359,7 @@ template <typename T> T *E(Mesh &m, int i) { return (T *)m.ev[i]; }
 // context to another side stream that waits for the fork point, join() brings the work back to the main
 // stream. The launches of one pass of a batch (one per transform length) touch different meshes, and most
 // of them fill a fraction of the GPU (48 .. 180 blocks), so one after another they leave it idle: 24 uneven
-// films took 3.13 ms of summed kernel time per RK4 step. 15 side streams: with 7 the launches of many small meshes
-// queued behind one another (16 films of 256 x 128 cells 249 us a step with 15, 304 with 7, 408 with 3, 218 in work
-// lists; 31 streams change no case by more than 7 % either way).
+// films took 3.13 ms of summed kernel time per RK4 step.
 struct Branches {
     bm_ctx *c;
     cudaStream_t main;
@@ -1365,7 +1382,7 @@ struct Branches {
             CK(cudaEventRecord(fork, main));
             return 0;
         }
-        const int k = turn++ % kSide;
+        const int k = turn++ % c->n_side;
         while ((int)c->side.size() <= k) {
             cudaStream_t s = nullptr;
             CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -1393,7 +1410,6 @@ struct Branches {
     }
     // an error path leaves the context on its own stream
     ~Branches() { c->stream = main; }
-    static constexpr int kSide = 15;
 };
 
 // ------------------------------------------------------------------ many meshes per launch

@@ -6,9 +6,9 @@
 // pencils of two columns: every butterfly, product and sign is one packed instruction for both, every global
 // access is 16 bytes, every shared access 16 (spectra) or 8 (kernel) bytes, and the addresses are shared.
 // A thread keeps its own component's spectrum in registers, so the 3 x 3 product reads the other two only.
-// Measured (film 512 x 512 x 8, Nz = 16, one launch): 45.8 -> 28.5 M warp instructions, 63.0 -> 57.1 us. At Nz = 32
-// the 128 value registers and 62 KB of spectra leave 9 warps per SM and the one-column form wins (150 against 160
-// us), so the tuner times both and FP64, which would need twice the registers, has none.
+// Measured (film 512 x 512 x 8, Nz = 16, one launch inside a step): 61.6 -> 58.1 us; warp instructions 41.9 -> 28.3 M.
+// At Nz = 32 the 128 value registers and 62 KB of spectra leave 9 warps per SM and the one-column form wins (137 against
+// 159 us), so the tuner times both and FP64, which would need twice the registers, has none.
 // Thread (c, p, wp), wp fastest; block = 3 components x the mirror pencils ky, Ny - ky x WP column pairs.
 #pragma once
 #include "kernels.h"
