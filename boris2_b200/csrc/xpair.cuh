@@ -9,8 +9,8 @@
 // inverse's first pass) and written (the forward's last pass) a thread's two lanes take mirror butterflies, so that
 // every element meets its mirror there and the spectrum crosses no shared memory.
 // Measured on the 512 x 512 x 16 film: stage launch 188 -> 168 us (of 503 MB: 3.0 TB/s), of which 176 -> 168 by the
-// mirror butterflies; 38.6 instead of 49.7 M warp instructions on its half. What bounds it now: the shared-memory
-// and L1 pipe and the latency of the cell rows behind it (long scoreboard 5 per issue).
+// mirror butterflies; 38.0 instead of 47.4 M warp instructions on its half. What bounds it now: load latency at a third
+// of the SM's warps (80 registers; long scoreboard 4.8 per issue, L1 52 % and DRAM 25 % busy).
 //
 // Shared line: c2 form for the passes (pair i at i + i / 8: conflict-free for every stride used), plain complex
 // order between the inverse and the forward transform, where element m is the pair of cells 2m, 2m + 1.
