@@ -174,6 +174,7 @@ struct bm_ctx {
     int kernels_per_step = 0;
     double *farq = nullptr;
     StepState host_st;
+    StepState *pin_st = nullptr;   // page-locked landing of the step state behind a field evaluation
     bool st_known = false;     // host_st equals the device's step state (nothing that writes it has run since)
     bool batched = false;       // many meshes per launch (work lists) instead of one launch per mesh
     int n_side = 7;             // side streams of a batched step's branches (branch_streams)
@@ -2344,15 +2345,20 @@ int run_T(bm_ctx *c, int steps)
     return 0;
 }
 
-// the end of a single field evaluation: waits for the stream and, where a launch can have set the error flag, reads
-// the step state with the same wait and reports it (the flag stays set until a new M, as after a run)
+// the end of a single field evaluation, in two parts around its copy to the host. Where a launch can have set the error
+// flag, the step state is read with the wait that the evaluation does anyway, and the flag reported (it stays set until
+// a new M, as after a run)
+int queue_state(bm_ctx *c)
+{
+    if (!c->st_known) CK(cudaMemcpyAsync(c->pin_st, c->st, sizeof(StepState), cudaMemcpyDeviceToHost, c->stream));
+    return 0;
+}
 int finish_field(bm_ctx *c)
 {
-    if (c->st_known) {
-        CK(cudaStreamSynchronize(c->stream));
-        return 0;
-    }
-    if (int rc = read_state(c)) return rc;
+    CK(cudaStreamSynchronize(c->stream));
+    if (c->st_known) return 0;
+    c->host_st = *c->pin_st;
+    c->st_known = true;
     return check_wait(c);
 }
 
@@ -2402,6 +2408,7 @@ int compute_field_T(bm_ctx *c, Mesh &m, int modules_mask, double *H)
     a.Hout = (T *)m.Hout;
     CKL(launch_stage<T>(a, c->stream), "heff");
     CKL(launch_planes_to_aos<T>(m.stage64, (const T *)m.Hout, m.n, c->stream), "planes_to_aos");
+    if (int rc = queue_state(c)) return rc;
     CK(cudaMemcpyAsync(H, m.stage64, sizeof(double) * 3 * m.n, cudaMemcpyDeviceToHost, c->stream));
     c->s1_dirty = true;
     return finish_field(c);
@@ -2642,6 +2649,7 @@ int bm_create(int device, bm_ctx **out)
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { delete c; return fail(BM_ECUDA, "stream"); }
     if (cudaMalloc(&c->st, sizeof(StepState)) != cudaSuccess) { delete c; return fail(BM_ENOMEM, "state"); }
     if (cudaMalloc(&c->farq, sizeof(double) * 6 * BM_FARQ_PER_COMP) != cudaSuccess) { delete c; return fail(BM_ENOMEM, "farq"); }
+    if (cudaMallocHost(&c->pin_st, sizeof(StepState)) != cudaSuccess) { delete c; return fail(BM_ENOMEM, "state"); }
     memset(&c->host_st, 0, sizeof(StepState));
     *out = c;
     return 0;
@@ -2656,6 +2664,7 @@ int bm_destroy(bm_ctx *c)
     for (auto &m : c->meshes) free_mesh(m);
     if (c->st) cudaFree(c->st);
     if (c->farq) cudaFree(c->farq);
+    if (c->pin_st) cudaFreeHost(c->pin_st);
     for (auto st : c->side) cudaStreamDestroy(st);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -3074,6 +3083,7 @@ int demag_device_T(bm_ctx *c, Mesh &m, const S *M, S *H, int add, double *energy
     double *dot = energy ? m.stage64 : nullptr;
     if (dot) CK(cudaMemsetAsync(dot, 0, sizeof(double), s));
     CKL((launch_planes_to_daos<S, T>(H, (const T *)m.Hout, m.n, add, M, dot, s)), "H out");
+    if (int rc = queue_state(c)) return rc;
     if (dot) {
         double d = 0.0;
         CK(cudaMemcpyAsync(&d, dot, sizeof(double), cudaMemcpyDeviceToHost, s));
