@@ -622,8 +622,8 @@ float time_launches(cudaStream_t s, F launch, int reps, float best = 0.f)
 template <typename T> bool tune_xv_ok(int LX, int xv)
 {
     // x-transform variants a length has: 0 always (the generic kernel where there is no register one), 4 (butterfly
-    // pairs) in FP32. Radix 16 (2, and 3 at the lower register cap) is not timed where FP32 has the pairs: over 34
-    // shapes with LX 256 .. 1024 it was never the fastest
+    // pairs) in FP32. Radix 16 (2, and 3 at the lower register cap) is not timed where FP32 has the pairs: in 40
+    // set-ups of 20 shapes with LX 256 .. 1024 it was never the fastest
     if (xv == 0) return true;
     if (xv == 1) return stage_reg_q(LX, 1) != 0;
     if (xv < 4 && sizeof(T) == 4 && stage_reg_q(LX, 4)) return false;
